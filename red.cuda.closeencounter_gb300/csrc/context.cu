@@ -71,6 +71,7 @@ struct rg_ctx {
     int* d_heavy = nullptr;  // per mixed tile: end of its heavy sources
     int tiles_cap = 0;
     void* d_split = nullptr;  // FP32 (hi, lo) positions of the mixed kernel
+    CertRows cert{};          // FP64 mode: the rows, scale and list of gravity_cert.cu
     float* d_rf = nullptr;    // FP32 radii of the mixed kernels' event screens
     unsigned int* d_smax = nullptr;  // the screens' maxima (split_positions)
     int* d_screen_slot = nullptr;    // per body: 0 for a light body, -1 for a heavy one
@@ -216,6 +217,10 @@ void free_all(rg_ctx* c)
     cudaFree(c->d_tiles);
     cudaFree(c->d_heavy);
     cudaFree(c->d_split);
+    cudaFree(c->cert.rows);
+    cudaFree(c->cert.scale);
+    cudaFree(c->cert.list);
+    cudaFree(c->cert.n_list);
     cudaFree(c->d_rf);
     cudaFree(c->d_smax);
     cudaFree(c->d_screen_slot);
@@ -350,7 +355,7 @@ int set_param_dev(rg_ctx* c, int i)
 enum {
     GROUP_PAIRPAR = 0,
     GROUP_ROWSEQ = 1,
-    GROUP_FEW_SERIAL = 2,
+    GROUP_FP64_ROWS = 2,
     GROUP_MIXED = 3,
     GROUP_DF_ROWSEQ = 4,  // mixed mode: the row kernel in double-float arithmetic
     GROUP_DF_FEW = 5,     // mixed mode: few heavy sinks in double-float arithmetic
@@ -405,7 +410,7 @@ void build_tiles(rg_ctx* c)
         for (int s = s0; s < s1; s += step) {
             c->tiles.push_back(Tile{s, std::min(s + step, s1), block == 0 ? src0 : 0, src1, 0, 0, block, 0});
             c->heavy_mx.push_back(kind == GROUP_MIXED ? std::min(n_heavy, src1) : 0);
-            if (kind == GROUP_FEW_SERIAL || kind == GROUP_DF_FEW) {
+            if (kind == GROUP_DF_FEW) {
                 c->few_row0.push_back(c->few_rows);
                 c->few_nsrc.push_back(src1);
                 for (int i = s; i < std::min(s + step, s1); i++) {
@@ -466,15 +471,18 @@ void build_tiles(rg_ctx* c)
             continue;
         }
         if (ns <= FEW_BLOCK_SINKS) {  // few sinks, many sources: exact serial row sums (same rows)
-            add_group(0, GROUP_FEW_SERIAL, b.s0, b.s1, b.src1, b.block, FEW_SINKS_MAX);
-            if (!(sym && b.block == 0)) {  // a symmetric plan's heavy rows come with its tiles
-                c->plan[1].push_back(c->plan[0].back());
-                c->plan[1].back().kind = GROUP_DF_FEW;
-            }
+            add_group(0, GROUP_FP64_ROWS, b.s0, b.s1, b.src1, b.block, 1);
+            if (!(sym && b.block == 0))  // a symmetric plan's heavy rows come with its tiles
+                add_group(1, GROUP_DF_FEW, b.s0, b.s1, b.src1, b.block, FEW_SINKS_MAX);
             continue;
         }
-        add_group(0, GROUP_PAIRPAR, b.s0, b.s1, b.src1, b.block, c->pairpar_S);
         const int light0 = b.block == 0 ? std::max(b.s0, std::min(n_heavy, b.s1)) : b.s0;
+        // the heavy rows' sums are as small as their terms, so their integers do not save the FP64
+        // terms (gravity_cert.cu): exact serial row sums, beside the light rows
+        // (small blocks: every row -- FP64_ROW_PAIRS)
+        const int pair0 = (int64_t)ns * b.src1 <= FP64_ROW_PAIRS ? b.s1 : (light0 - b.s0 <= FEW_BLOCK_SINKS ? light0 : b.s0);
+        add_group(0, GROUP_FP64_ROWS, b.s0, pair0, b.src1, b.block, 1);
+        add_group(0, GROUP_PAIRPAR, pair0, b.s1, b.src1, b.block, c->pairpar_S);
         add_group(1, GROUP_DF_FEW, b.s0, light0, b.src1, b.block, FEW_SINKS_MAX);
         add_group(1, GROUP_MIXED, light0, b.s1, b.src1, b.block, MIXED_SINKS_PER_TILE);
     }
@@ -614,7 +622,7 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
         g.astro = c->d_astro;
         g.astro_stride = (long long)cap;
     }
-    bool split_done = false;
+    bool split_done = false, cert = false;
     // with a mixed group, the double-float row groups (a few sinks: star, giants) run on a
     // side stream beside it: they write other rows and append events atomically
     bool fork = false;
@@ -638,7 +646,7 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
     bool fork_few = false;
     if (c->gravity_mode == RG_GRAVITY_FP64) {
         bool few = false, other = false;
-        for (const auto& gr : c->plan[0]) (gr.kind == GROUP_FEW_SERIAL ? few : other) = true;
+        for (const auto& gr : c->plan[0]) (gr.kind == GROUP_FP64_ROWS ? few : other) = true;
         fork_few = few && other;
     }
     if (fork_few) {
@@ -650,18 +658,27 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
         g.n_tiles = gr.n;
         switch (gr.kind) {
         case GROUP_PAIRPAR:
-            rc = launch_grav_fp64_pairpar(g, c->pairpar_S, c->st);
+            if (c->frame == RG_FRAME_ASTRO) {
+                rc = launch_grav_fp64_pairpar(g, c->pairpar_S, c->st);
+                c->n_kernels++;
+                break;
+            }
+            if (!split_done) {
+                rc = launch_cert_prep(g, nullptr, nullptr, 1, c->n_total(), c->cert, c->st);
+                split_done = true;
+                c->n_kernels++;
+            }
+            if (!rc) rc = launch_grav_fp64_cert(g, c->cert, c->pairpar_S, c->st);
             c->n_kernels++;
+            cert = true;
             break;
         case GROUP_ROWSEQ:
             rc = launch_grav_fp64_rowseq(g, c->st);
             c->n_kernels++;
             break;
-        case GROUP_FEW_SERIAL:
-            rc = launch_grav_fp64_few(g, c->d_few_row0 + gr.off, gr.max_src, c->d_terms, c->few_rows, c->few_pitch,
-                                      c->d_row_sink, c->d_row_nsrc, nullptr, gr.row_base, gr.rows,
-                                      fork_few ? c->st2 : c->st);
-            c->n_kernels += 2;
+        case GROUP_FP64_ROWS:
+            rc = launch_grav_fp64_rows(g, fork_few ? c->st2 : c->st);
+            c->n_kernels++;
             break;
         case GROUP_DF_ROWSEQ:
         case GROUP_DF_FEW:
@@ -737,6 +754,10 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
             break;
         }
         if (rc) break;
+    }
+    if (cert && !rc) {  // the rows the pair-parallel kernel left over
+        rc = launch_grav_fp64_list(g, c->cert, c->st);
+        c->n_kernels++;
     }
     if (fork || fork_few) {  // joined on every path, so that no row kernel outlives the call's stream order
         RG_CUDA_CHECK(cudaEventRecord(c->ev_join, c->st2));
@@ -1536,24 +1557,20 @@ int rg_device_count(void)
     return n;
 }
 
-// The default sinks per pair-parallel CTA: every CTA of the self-interacting block runs all of
-// its sources, so a launch takes (waves of resident CTAs) x (one CTA's time, proportional to
-// S); the S of the candidate set with the fewest wave-sinks, the larger S on a tie (fewer
-// barriers per pair).  16 385 sinks on 152 SMs x 3 CTAs: S = 36, one wave of 456 CTAs.
-// rg_autotune times the candidates instead.
-static int wave_best_sinks(const rg_ctx* c)
+// The default sinks per pair-parallel tile.  Barycentric frame: a tile's sinks are shared out
+// over independent warps (gravity_cert.cu), so only the last tile's unused warps depend on it.
+// Astrocentric frame: every CTA of the block runs all of its sources, so a launch takes (waves of
+// resident CTAs) x (one CTA's time, proportional to S); the S of the candidate set with the
+// fewest wave-sinks, the larger S on a tie (fewer barriers per pair).  rg_autotune times the
+// candidates instead.
+static int default_sinks(const rg_ctx* c)
 {
-    const int ns = c->n_si() - (c->frame == RG_FRAME_ASTRO ? 1 : 0);
-    if (ns <= 0) return 16;
+    const int ns = c->n_si() - 1;
+    if (c->frame != RG_FRAME_ASTRO || ns <= 0) return 16;
     const long long slots = (long long)std::max(c->n_sm, 1) * RG_PAIRPAR_RESIDENT;
-    static const int astro_s[] = {8, 16, 32};
-    static const int bary_s[] = {8, 12, 16, 18, 24, 32, 36};
-    const int* cand = c->frame == RG_FRAME_ASTRO ? astro_s : bary_s;
-    const int nc = c->frame == RG_FRAME_ASTRO ? 3 : 7;
     int best = 16;
     long long best_cost = -1;
-    for (int k = 0; k < nc; k++) {
-        const int S = cand[k];
+    for (const int S : {8, 16, 32}) {
         const long long ctas = (ns + S - 1) / S;
         const long long cost = (ctas + slots - 1) / slots * S;
         if (best_cost < 0 || cost < best_cost || (cost == best_cost && S > best)) {
@@ -1631,6 +1648,11 @@ static int create_impl(const rg_counts_t* n, const rg_vec_t* r, const rg_vec_t* 
     chk(dalloc(&c->d_part, (size_t)5 * nt));
     chk(dalloc(&c->d_records, (size_t)8 * nt));
     chk(dalloc((char**)&c->d_split, SPLIT_POS_BYTES * (size_t)nt));
+    c->cert.stride = cert_stride(nt, 1);
+    chk(dalloc(&c->cert.rows, (size_t)(8 * c->cert.stride)));
+    chk(dalloc(&c->cert.scale, 8));
+    chk(dalloc(&c->cert.list, nt));
+    chk(dalloc(&c->cert.n_list, 1));
     chk(dalloc(&c->d_rf, nt));
     chk(dalloc(&c->d_smax, SCREEN_MAX_WORDS));
     chk(dalloc(&c->d_screen_slot, nt));
@@ -1723,7 +1745,7 @@ static int create_impl(const rg_counts_t* n, const rg_vec_t* r, const rg_vec_t* 
         delete c;
         return rc;
     }
-    c->pairpar_S = wave_best_sinks(c);
+    c->pairpar_S = default_sinks(c);
     build_tiles(c);
     *out = c;
     return RG_OK;

@@ -168,5 +168,10 @@ __device__ __forceinline__ void split_coord(double v, float& hi, float& lo)
     }
 }
 
+// a body's coordinates and mass, each split into FP32 (hi, lo)
+struct SplitPos {
+    float4 xy;  // x_hi, x_lo, y_hi, y_lo
+    float4 zm;  // z_hi, z_lo, m_hi, m_lo
+};
 
 }  // namespace redgb

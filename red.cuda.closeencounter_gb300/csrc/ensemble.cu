@@ -814,6 +814,8 @@ struct rg_ens {
     int* d_id = nullptr;
     int* d_type = nullptr;
     void* d_split = nullptr;
+    CertRows cert{};  // FP64 mode: the rows, scales and list of gravity_cert.cu
+    int max_n = 0;  // bodies of the largest disk
     float* d_rf = nullptr;  // FP32 radii of the mixed kernels' event screens
     float2* d_mass_f2 = nullptr;  // the split masses (the symmetric kernel's later stages)
     unsigned int* d_smax = nullptr;  // the screens' maxima per disk (split_positions)
@@ -950,7 +952,7 @@ constexpr long long ATTEMPT_CHUNK = 4096;  // attempts per graph launch at most
 enum {
     GROUP_PAIRPAR = 0,
     GROUP_ROWSEQ = 1,
-    GROUP_FEW_SERIAL = 2,
+    GROUP_FP64_ROWS = 2,
     GROUP_MIXED = 3,
     GROUP_DF_ROWSEQ = 4,
     GROUP_DF_FEW = 5,
@@ -976,6 +978,7 @@ void free_all(rg_ens* e)
     if (e->exec) cudaGraphExecDestroy(e->exec);
     if (e->graph) cudaGraphDestroy(e->graph);
     void* ptrs[] = {e->d_y, e->d_yout, e->d_P, e->d_mass, e->d_radius, e->d_rho, e->d_id, e->d_type, e->d_split,
+                    e->cert.rows, e->cert.scale, e->cert.list, e->cert.n_list,
                     e->d_partial, e->d_thr, e->d_status, e->d_active, e->d_active_f0, e->d_acc, e->d_ej,
                     e->d_sys_events, e->d_maxbits, e->d_t, e->d_tprev, e->d_tstop, e->d_dt_try, e->d_dt_did,
                     e->d_ntried, e->d_npassed, e->d_nfailed, e->d_attempt, e->d_acc_attempt, e->d_nf0, e->d_stiles,
@@ -1088,6 +1091,12 @@ void build_gravity_plan(rg_ens* e)
         hv[1][GROUP_DF_SYM].assign(by[1][GROUP_DF_SYM].size(), 0);
         for (size_t k = 0; k < sym_systems.size(); k++) sym_parts[sym_systems[k].sys] = parts[k];
     }
+    int64_t block_pairs = 0;  // of the blocks with many sinks and many sources, all disks
+    for (int s = 0; s < e->n_sys; s++) {
+        const int64_t nsi = e->n_si(s), nm = e->n_massive(s), nt = e->ntot[s];
+        for (const auto& k : {std::make_pair(nsi, nm), std::make_pair(nm - nsi, nsi), std::make_pair(nt - nm, nm)})
+            if (k.second > e->rowseq_max_src && k.first > ENS_FEW_BLOCK) block_pairs += k.first * k.second;
+    }
     for (int s = 0; s < e->n_sys; s++) {
         const int b = e->base[s];
         const int nsi = e->n_si(s), nm = e->n_massive(s), nt = e->ntot[s];
@@ -1110,12 +1119,15 @@ void build_gravity_plan(rg_ens* e)
                 if (!(sym[s] && k.block == 1))  // a symmetric system's light rows: the segments above
                     add(1, GROUP_DF_ROWSEQ, k.s0, k.s1, k.src1, k.block, 128);
             } else if (k.s1 - k.s0 <= ENS_FEW_BLOCK) {
-                add(0, GROUP_FEW_SERIAL, k.s0, k.s1, k.src1, k.block, FEW_SINKS_MAX);
+                add(0, GROUP_FP64_ROWS, k.s0, k.s1, k.src1, k.block, 1);
                 if (!(sym[s] && k.block == 0))  // a symmetric system's heavy rows come with its tiles
                     add(1, GROUP_DF_FEW, k.s0, k.s1, k.src1, k.block, FEW_SINKS_MAX);
             } else {
-                add(0, GROUP_PAIRPAR, k.s0, k.s1, k.src1, k.block, e->pairpar_S);  // S sinks per CTA and tile
                 const int light0 = k.block == 0 ? std::max(k.s0, std::min(n_heavy, k.s1)) : k.s0;
+                // heavy rows: exact serial sums (their terms are as large as the sums, gravity_cert.cu)
+                const int pair0 = block_pairs <= FP64_ROW_PAIRS ? k.s1 : (light0 - k.s0 <= ENS_FEW_BLOCK ? light0 : k.s0);
+                add(0, GROUP_FP64_ROWS, k.s0, pair0, k.src1, k.block, 1);
+                add(0, GROUP_PAIRPAR, pair0, k.s1, k.src1, k.block, e->pairpar_S);  // S sinks per tile
                 add(1, GROUP_DF_FEW, k.s0, light0, k.src1, k.block, FEW_SINKS_MAX);
                 add(1, GROUP_MIXED, light0, k.s1, k.src1, k.block, MIXED_SINKS_PER_TILE);
             }
@@ -1130,7 +1142,7 @@ void build_gravity_plan(rg_ens* e)
             for (size_t k = 0; k < T.size(); k++) {
                 e->tiles.push_back(T[k]);
                 e->heavy.push_back(hv[mode][kind][k]);
-                if (kind == GROUP_FEW_SERIAL || kind == GROUP_DF_FEW) {
+                if (kind == GROUP_DF_FEW) {
                     e->few_row0.push_back(e->few_rows);
                     const int nsrc = T[k].src_end - T[k].src_begin;
                     for (int i = T[k].sink_begin; i < T[k].sink_end; i++) {
@@ -1285,7 +1297,7 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
         g.smax = e->d_smax;
     }
     const auto& plan = e->plan[e->gravity_mode == RG_GRAVITY_MIXED ? 1 : 0];
-    bool split_done = false;
+    bool split_done = false, cert = false;
     // a later stage of the attempt needs only the coordinates split again: the step start's
     // split wrote the masses and radii, which change only at events (after the attempt); when
     // the symmetric kernel is the only one, it splits the coordinates itself (from the FP64
@@ -1323,12 +1335,20 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
         g.tiles = e->d_tiles + gr.off;
         g.n_tiles = gr.n;
         switch (gr.kind) {
-        case GROUP_PAIRPAR: rc = launch_grav_fp64_pairpar(g, e->pairpar_S, e->st); e->n_kernels++; break;
+        case GROUP_PAIRPAR:
+            if (!split_done) {
+                rc = launch_cert_prep(g, e->d_base, e->d_ntot, e->n_sys, e->max_n, e->cert, e->st);
+                split_done = true;
+                e->n_kernels++;
+            }
+            if (!rc) rc = launch_grav_fp64_cert(g, e->cert, e->pairpar_S, e->st);
+            e->n_kernels++;
+            cert = true;
+            break;
         case GROUP_ROWSEQ: rc = launch_grav_fp64_rowseq(g, row_st); e->n_kernels++; break;
-        case GROUP_FEW_SERIAL:
-            rc = launch_grav_fp64_few(g, e->d_few_row0 + gr.off, gr.max_src, e->d_terms, e->few_rows, e->few_pitch,
-                                      e->d_row_sink, e->d_row_nsrc, e->d_row_sys, gr.row_base, gr.rows, e->st);
-            e->n_kernels += 2;
+        case GROUP_FP64_ROWS:
+            rc = launch_grav_fp64_rows(g, e->st);
+            e->n_kernels++;
             break;
         case GROUP_DF_ROWSEQ:
         case GROUP_DF_FEW:
@@ -1376,6 +1396,10 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
             break;
         }
         if (rc) break;
+    }
+    if (cert && !rc) {  // the rows the pair-parallel kernel left over
+        rc = launch_grav_fp64_list(g, e->cert, e->st);
+        e->n_kernels++;
     }
     if (fork) {  // join (also after an error: a capture must not end with the side stream open)
         RG_CUDA_CHECK(cudaEventRecord(e->ev_join, e->st2));
@@ -1732,6 +1756,16 @@ int create_impl(int n_sys, const rg_counts_t* counts, const rg_vec_t* r, const r
     chk(dalloc(&e->d_type, nt));
     chk(dalloc(&e->d_base_of, nt));
     chk(dalloc((char**)&e->d_split, SPLIT_POS_BYTES * nt));
+    bool pairpar = false;  // a disk with a block for the pair-parallel kernel
+    for (int s = 0; s < n_sys; s++) {
+        e->max_n = std::max(e->max_n, e->ntot[s]);
+        pairpar = pairpar || e->n_si(s) > ENS_FEW_BLOCK || e->ntot[s] - e->n_massive(s) > ENS_FEW_BLOCK;
+    }
+    e->cert.stride = cert_stride((int)nt, n_sys);
+    chk(dalloc(&e->cert.rows, pairpar ? (size_t)(8 * e->cert.stride) : 1));
+    chk(dalloc(&e->cert.scale, 8 * ns));
+    chk(dalloc(&e->cert.list, pairpar ? nt : 1));
+    chk(dalloc(&e->cert.n_list, 1));
     chk(dalloc(&e->d_rf, nt));
     chk(dalloc(&e->d_mass_f2, nt));
     chk(dalloc(&e->d_smax, (size_t)SCREEN_MAX_WORDS * ns));

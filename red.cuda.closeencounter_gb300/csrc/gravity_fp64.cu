@@ -19,72 +19,19 @@
 // 1027 sources in the planetesimal disk), which thread-per-sink scheduling cannot.
 // The row-serial kernel (thread per sink) serves blocks with few sources per sink
 // (planetesimals x 3 massive bodies).  Sources are staged through shared memory in both.
+#include <atomic>
 #include <string>
 
 #include "../../include/redgb.h"
 #include "common.cuh"
 #include "exact_fp64.h"
 #include "kernels.h"
+#include "pair_fp64.cuh"
+#include "row_sum.h"
 
 namespace redgb {
 
 int set_error(int code, const std::string& msg);
-
-struct PairOut {
-    double tx, ty, tz;
-};
-
-// One (sink, source) pair: the term added to a_i and the event tests of pp_disk.cu:265
-// (radius criterion) and of the mutual Hill sphere (cube form, no cube root).
-__device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, int i, int j, double xi, double yi,
-                                          double zi, double Ri, double mi, double rhoi, double xj, double yj,
-                                          double zj, double mj, double Rj, double rhoj, PairOut& o)
-{
-    const double dx = xj - xi;
-    const double dy = yj - yi;
-    const double dz = zj - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double d = rn_sqrt(r2);         // sqrt.rn, computed on the integer pipes
-    const double w = rn_div(mj, d * r2);  // div.rn, likewise (exact_fp64.h)
-    o.tx = w * dx;
-    o.ty = w * dy;
-    o.tz = w * dz;
-    const int li = i - tile.base, lj = j - tile.base;
-    bool rad = g.record && li > 0 && li > lj && d < tile_f_rad(g, tile) * (Ri + Rj);
-    bool hill = false;
-    if (g.hill && tile.block != 2 && li > 0 && li > lj && lj > 0) {
-        const double h = 0.5 * (rhoi + rhoj);
-        const double lhs = d * d * d;
-        const double rhs = ((g.hill_f3 * (mi + mj)) / (3.0 * g.mass[tile.base])) * (h * h * h);
-        hill = lhs < rhs;
-    }
-    if (rad || hill) {
-        for (int kind = 0; kind < 2; kind++) {
-            if (!(kind == 0 ? rad : hill)) continue;
-            const EventBuf& eb = kind == 0 ? g.ev : g.hv;
-            unsigned int slot = atomicAdd(eb.count, 1u);
-            if (kind == 0 && g.sys_events) atomicAdd(&g.sys_events[tile.sys], 1u);
-            if (slot < eb.cap) {
-                DevEvent* e = &eb.rec[slot];
-                e->seq = record_seq(g, tile, kind);
-                e->kind = kind;
-                e->i = i;
-                e->j = j;
-                e->sys = tile.sys;
-                e->pad = 0;
-                e->d = d;
-                e->t = g.sys_t ? g.sys_t[tile.sys] : 0.0;
-                const int b0 = tile.base;
-                e->ri[0] = xi; e->ri[1] = yi; e->ri[2] = zi;
-                e->rj[0] = xj; e->rj[1] = yj; e->rj[2] = zj;
-                e->vi[0] = g.vx[i]; e->vi[1] = g.vy[i]; e->vi[2] = g.vz[i];
-                e->vj[0] = g.vx[j]; e->vj[1] = g.vy[j]; e->vj[2] = g.vz[j];
-                e->r0[0] = g.px[b0]; e->r0[1] = g.py[b0]; e->r0[2] = g.pz[b0];
-                e->v0[0] = g.vx[b0]; e->v0[1] = g.vy[b0]; e->v0[2] = g.vz[b0];
-            }
-        }
-    }
-}
 
 // ---------------------------------------------------------------------------------------
 // Pair-parallel kernel: CTA = S sinks, source tiles of J = 1024 / S.  ASTRO: the
@@ -243,119 +190,70 @@ __global__ void star_distance(const double* __restrict__ x, const double* __rest
 }
 
 // ---------------------------------------------------------------------------------------
-// Few-sink path: blocks with a handful of sinks and many sources (the star and giants
-// of a planetesimal disk).  Kernel A spreads the pair terms of up to FEW_MAX sinks over
-// the whole GPU, one thread per source, into a terms buffer (3 x rows x n_src); kernel B
-// adds each row in ascending source order -- one thread per (sink, component), which is
-// the reference's serial sum -- or, for the mixed-precision kernel's heavy rows, as a
-// compensated tree reduction.
-constexpr int FEW_MAX = 8;
+// Row path: rows whose sums need every bit of their terms -- blocks with a handful of sinks and
+// many sources (the star and giants of a planetesimal disk), and the rows gravity_cert.cu leaves
+// over.  One CTA per row: eight warps compute the exact terms of a chunk of sources into shared
+// memory while three others, one per component, add the chunk before it in ascending source
+// order (warp_row_sum, row_sum.h).
+//
+// Bound: a chunk of 1152 pairs is 36 warps x 12 FP64 operations x 16 cycles of the SM's FP64 pipe
+// (6.9 k cycles), its sums 4-12 k cycles of latency beside them; the serial additions they replace
+// took 71 cycles per term.
+constexpr int ROW_TERM_WARPS = 8;
+constexpr int ROW_WARPS = 3 + ROW_TERM_WARPS;
+constexpr int ROW_CHUNK = 32 * ROW_SEG_MAX;
+constexpr int ROW_PITCH = 32 * (ROW_SEG_MAX | 1);
 
-struct FewArgs {
-    GravArgs g;
-    const int* tile_row0;  // first row of each tile in the terms buffer
-    double* terms;         // 3 x rows x pitch
-    int rows;              // rows of the buffer
-    long long pitch;       // >= largest source count
+struct RowSmem {
+    double term[2][3][ROW_PITCH];
+    uint32_t codes[3][32 * ROW_SEG_MAX];
 };
 
-__global__ void __launch_bounds__(256) grav_fp64_few_terms(FewArgs a)
+// LIST: the rows *n_list of `list` (part: components to add), without event tests
+template <bool LIST>
+__global__ void __launch_bounds__(32 * ROW_WARPS) grav_fp64_rows(GravArgs g, const Tile* list, const unsigned int* n_list)
 {
-    const GravArgs& g = a.g;
-    const Tile tile = g.tiles[blockIdx.y];
-    if (g.sys_active && !g.sys_active[tile.sys]) return;
-    if ((int)(blockIdx.x * blockDim.x) >= tile.src_end - tile.src_begin) return;
-    const int row0 = a.tile_row0[blockIdx.y];
-    const int q = blockIdx.x * blockDim.x + threadIdx.x;  // source offset within the tile
-    const int j = tile.src_begin + q;
-    __shared__ double sx[FEW_MAX], sy[FEW_MAX], sz[FEW_MAX], sR[FEW_MAX], sm[FEW_MAX], srho[FEW_MAX];
-    __shared__ int sact[FEW_MAX];
-    const int ns = tile.sink_end - tile.sink_begin;
-    if (threadIdx.x < ns) {
-        const int i = tile.sink_begin + threadIdx.x;
-        sx[threadIdx.x] = g.px[i]; sy[threadIdx.x] = g.py[i]; sz[threadIdx.x] = g.pz[i];
-        sR[threadIdx.x] = g.radius[i]; sm[threadIdx.x] = g.mass[i];
-        srho[threadIdx.x] = g.hill ? g.rho[i] : 0.0;
-        sact[threadIdx.x] = 0 < g.id[i];
-    }
-    __syncthreads();
-    if (j >= tile.src_end) return;
-    const double xj = g.px[j], yj = g.py[j], zj = g.pz[j], mj = g.mass[j], Rj = g.radius[j];
-    const double rhoj = g.hill ? g.rho[j] : 0.0;
-    const bool src_ok = 0 <= g.id[j];
-    const long long plane = (long long)a.rows * a.pitch;
-    for (int s = 0; s < ns; s++) {
-        const int i = tile.sink_begin + s;
-        PairOut o{0.0, 0.0, 0.0};
-        if (sact[s] && src_ok && j != i)
-            pair_term(g, tile, i, j, sx[s], sy[s], sz[s], sR[s], sm[s], srho[s], xj, yj, zj, mj, Rj, rhoj, o);
-        const long long e = (long long)(row0 + s) * a.pitch + q;
-        a.terms[e] = o.tx;
-        a.terms[plane + e] = o.ty;
-        a.terms[2 * plane + e] = o.tz;
-    }
-}
-
-struct FewSumArgs {
-    const double* terms;
-    int rows;         // rows of the whole buffer
-    int row0, nrows;  // the rows this launch sums
-    long long pitch;
-    const int* row_sink;   // sink index of each row
-    const int* row_nsrc;   // sources of each row
-    const int* row_sys;    // system of each row (ensembles) or nullptr
-    const int* sys_active;
-    double* ax;
-    double* ay;
-    double* az;
-};
-
-// exact: one warp per (row, component).  The warp streams the row through shared memory
-// in coalesced chunks (the next chunk's loads are in flight while the current one is added)
-// and adds the terms in ascending source order with the bits of the reference's serial sum:
-// warp_serial_sum (exact_fp64.h) takes 32 terms per pass on the integer pipes, where a chain
-// of dependent FP64 additions would wait on GB300's FP64 latency for each term.
-constexpr int SUM_CHUNK = 256;
-
-__global__ void __launch_bounds__(128) few_sum_serial(FewSumArgs a)
-{
-    __shared__ double buf[4][2][SUM_CHUNK];
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    RowSmem& M = *reinterpret_cast<RowSmem*>(row_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int t = blockIdx.x * 4 + warp;
-    if (t >= 3 * a.nrows) return;
-    const int comp = t / a.nrows, row = a.row0 + t % a.nrows;
-    if (a.sys_active && !a.sys_active[a.row_sys[row]]) return;
-    const double* T = a.terms + ((long long)comp * a.rows + row) * a.pitch;
-    const int n = a.row_nsrc[row];
-    double (*B)[SUM_CHUNK] = buf[warp];
-    double reg[SUM_CHUNK / 32];
-    auto load = [&](int c0) {
-#pragma unroll
-        for (int k = 0; k < SUM_CHUNK / 32; k++) {
-            const int q = c0 + k * 32 + lane;
-            reg[k] = q < n ? T[q] : 0.0;
+    const int n_rows = LIST ? (int)*n_list : g.n_tiles;
+    for (int row = blockIdx.x; row < n_rows; row += gridDim.x) {
+        const Tile tile = LIST ? list[row] : g.tiles[row];
+        if (g.sys_active && !g.sys_active[tile.sys]) continue;
+        const int comps = LIST ? tile.part : 7;
+        const int i = tile.sink_begin;
+        const bool active = 0 < g.id[i];
+        const double xi = g.px[i], yi = g.py[i], zi = g.pz[i];
+        const double Ri = LIST ? 0.0 : g.radius[i], mi = LIST ? 0.0 : g.mass[i], rhoi = !LIST && g.hill ? g.rho[i] : 0.0;
+        double acc = 0.0;
+        const int n = tile.src_end - tile.src_begin;
+        const int chunks = (n + ROW_CHUNK - 1) / ROW_CHUNK;
+        for (int c = 0; c <= chunks; c++) {
+            if (c < chunks && (c == 0 || warp >= 3)) {  // terms of chunk c (the first one: by every warp)
+                const int q0 = c * ROW_CHUNK, m = min(ROW_CHUNK, n - q0);
+                const int seg = (m + 31) / 32, pitch = seg | 1;
+                const int w0 = c == 0 ? 0 : 3, nw = ROW_WARPS - w0;
+                for (int q = (warp - w0) * 32 + lane; q < m; q += 32 * nw) {
+                    const int j = tile.src_begin + q0 + q;
+                    const double xj = g.px[j], yj = g.py[j], zj = g.pz[j], mj = g.mass[j];
+                    PairOut o{0.0, 0.0, 0.0};
+                    if (active && j != i && 0 <= g.id[j])
+                        pair_term<!LIST>(g, tile, i, j, xi, yi, zi, Ri, mi, rhoi, xj, yj, zj, mj, LIST ? 0.0 : g.radius[j],
+                                         !LIST && g.hill ? g.rho[j] : 0.0, o);
+                    const int at = q / seg * pitch + q % seg;
+                    M.term[c & 1][0][at] = o.tx;
+                    M.term[c & 1][1][at] = o.ty;
+                    M.term[c & 1][2][at] = o.tz;
+                }
+            }
+            if (c > 0 && warp < 3 && (comps >> warp & 1)) {
+                const int m = min(ROW_CHUNK, n - (c - 1) * ROW_CHUNK);
+                const int seg = (m + 31) / 32;
+                acc = warp_row_sum(acc, M.term[(c - 1) & 1][warp], seg, seg | 1, m, M.codes[warp]);
+            }
+            __syncthreads();
         }
-    };
-    double acc = 0.0;
-    SerialSumState sst{0, 0};
-    int cur = 0;
-    load(0);
-    for (int c0 = 0; c0 < n; c0 += SUM_CHUNK) {
-#pragma unroll
-        for (int k = 0; k < SUM_CHUNK / 32; k++) B[cur][k * 32 + lane] = reg[k];
-        __syncwarp();
-        if (c0 + SUM_CHUNK < n) load(c0 + SUM_CHUNK);
-        const int m = min(SUM_CHUNK, n - c0);
-        for (int b = 0; b < m; b += 32) {
-            const int mb = min(32, m - b);
-            acc = warp_serial_sum(acc, &B[cur][b], mb, sst);
-        }
-        __syncwarp();
-        cur ^= 1;
-    }
-    if (lane == 0) {
-        double* out = comp == 0 ? a.ax : (comp == 1 ? a.ay : a.az);
-        out[a.row_sink[row]] = acc;
+        if (warp < 3 && lane == 0 && (comps >> warp & 1)) (warp == 0 ? g.ax : warp == 1 ? g.ay : g.az)[i] = acc;
     }
 }
 
@@ -400,17 +298,6 @@ int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st)
         case 32: grav_fp64_pairpar<32, 8, true><<<g.n_tiles, 256, 0, st>>>(g); break;
         default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 16 or 32 in the astrocentric frame");
         }
-    } else {
-        switch (S) {
-        case 8: grav_fp64_pairpar<8, 32, false><<<g.n_tiles, 256, 0, st>>>(g); break;
-        case 12: grav_fp64_pairpar<12, 21, false><<<g.n_tiles, 252, 0, st>>>(g); break;
-        case 16: grav_fp64_pairpar<16, 16, false><<<g.n_tiles, 256, 0, st>>>(g); break;
-        case 18: grav_fp64_pairpar<18, 14, false><<<g.n_tiles, 252, 0, st>>>(g); break;
-        case 24: grav_fp64_pairpar<24, 10, false><<<g.n_tiles, 240, 0, st>>>(g); break;
-        case 32: grav_fp64_pairpar<32, 8, false><<<g.n_tiles, 256, 0, st>>>(g); break;
-        case 36: grav_fp64_pairpar<36, 7, false><<<g.n_tiles, 252, 0, st>>>(g); break;
-        default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 12, 16, 18, 24, 32 or 36");
-        }
     }
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
@@ -433,23 +320,36 @@ int launch_grav_fp64_rowseq(const GravArgs& g, cudaStream_t st)
     return 0;
 }
 
-// Few-sink tiles (at most FEW_MAX sinks each) -> terms -> exact serial row sums, one launch
-// each for all tiles of the group.  Rows are numbered tile by tile; tile_row0 (device) gives
-// each tile's first row, max_src bounds the tiles' source counts, and the row arrays
-// (dev_row_sink, dev_row_nsrc, dev_row_sys) are on the device.
-int launch_grav_fp64_few(const GravArgs& g, const int* tile_row0, int max_src, double* terms, int rows,
-                         long long pitch, const int* dev_row_sink, const int* dev_row_nsrc, const int* dev_row_sys,
-                         int group_row0, int group_rows, cudaStream_t st)
+// the row kernels' shared memory: a per-device attribute, set once per device (setting it again
+// from another thread is harmless)
+static int row_attributes()
 {
-    if (g.n_tiles <= 0 || rows <= 0 || group_rows <= 0 || max_src <= 0) return 0;
-    FewArgs a{g, tile_row0, terms, rows, pitch};
-    // 256 sources per CTA, or 64 when that would leave most SMs idle (one disk's few heavy rows)
-    const int nt = (long long)((max_src + 255) / 256) * g.n_tiles < 2 * NUM_SMS_HINT ? 64 : 256;
-    grav_fp64_few_terms<<<dim3((max_src + nt - 1) / nt, g.n_tiles), nt, 0, st>>>(a);
+    static std::atomic<bool> attr_set[64];
+    int dev = 0;
+    RG_CUDA_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
+        const int smem = (int)sizeof(RowSmem);
+        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
+    }
+    return 0;
+}
+
+int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st)
+{
+    if (g.n_tiles <= 0) return 0;
+    if (const int rc = row_attributes()) return rc;
+    grav_fp64_rows<false><<<g.n_tiles, 32 * ROW_WARPS, sizeof(RowSmem), st>>>(g, nullptr, nullptr);
     RG_CUDA_CHECK(cudaGetLastError());
-    FewSumArgs b{terms, rows, group_row0, group_rows, pitch, dev_row_sink, dev_row_nsrc, dev_row_sys, g.sys_active,
-                 g.ax, g.ay, g.az};
-    few_sum_serial<<<(3 * group_rows + 3) / 4, 128, 0, st>>>(b);
+    return 0;
+}
+
+int launch_grav_fp64_list(const GravArgs& g, const CertRows& cr, cudaStream_t st)
+{
+    if (const int rc = row_attributes()) return rc;
+    // as many CTAs as are resident (three per SM); the list's length is known on the device
+    grav_fp64_rows<true><<<3 * NUM_SMS_HINT, 32 * ROW_WARPS, sizeof(RowSmem), st>>>(g, cr.list, cr.n_list);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

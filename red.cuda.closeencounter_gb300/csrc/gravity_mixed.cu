@@ -39,11 +39,6 @@ namespace redgb {
 
 int set_error(int code, const std::string& msg);
 
-struct SplitPos {
-    float4 xy;  // x_hi, x_lo, y_hi, y_lo
-    float4 zm;  // z_hi, z_lo, m_hi, m_lo
-};
-
 // inactive bodies (id < 0, pp_disk.cu:242) get mass 0 here, so the pair loop needs no
 // per-pair activity test: their terms vanish.  Coordinates beyond 1e15 AU are clamped
 // (split_coord, dfloat.cuh).

@@ -75,14 +75,34 @@ int launch_energy(const EnergyArgs& a, cudaStream_t st);
 
 // resident pair-parallel CTAs per SM (the kernels are built for it: 80 registers, 256 threads)
 constexpr int RG_PAIRPAR_RESIDENT = 3;
-int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st);
+int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st);  // astrocentric frame
+// barycentric frame (gravity_cert.cu): launch_cert_prep writes an evaluation's rows and scales
+// (sys_base, sys_n: each system's first body and body count, or nullptr: one system of max_n
+// bodies), launch_grav_fp64_cert the tiles' sums (S: sinks per tile)
+// except those it lists, which launch_grav_fp64_list (gravity_fp64.cu) then adds
+struct CertRows {
+    float* rows;       // 8 FP32 rows of `stride` (cert_stride)
+    long long stride;
+    float* scale;      // 8 per system
+    Tile* list;        // rows left over: one sink each, part = its components (bits); one slot per body
+    unsigned int* n_list;
+};
+long long cert_stride(int n, int n_sys);
+int launch_cert_prep(const GravArgs& g, const int* sys_base, const int* sys_n, int n_sys, int max_n, const CertRows& cr,
+                     cudaStream_t st);
+int launch_grav_fp64_cert(const GravArgs& g, const CertRows& cr, int S, cudaStream_t st);
+int launch_grav_fp64_list(const GravArgs& g, const CertRows& cr, cudaStream_t st);
 int launch_astro_terms(const double* x, const double* y, const double* z, const double* mass, int n, double m_star,
                        double* out, long long stride, cudaStream_t st);
 int launch_grav_fp64_rowseq(const GravArgs& g, cudaStream_t st);
-constexpr int FEW_SINKS_MAX = 8;  // sinks per few-sink tile
-int launch_grav_fp64_few(const GravArgs& g, const int* tile_row0, int max_src, double* terms, int rows,
-                         long long pitch, const int* dev_row_sink, const int* dev_row_nsrc, const int* dev_row_sys,
-                         int group_row0, int group_rows, cudaStream_t st);
+constexpr int FEW_SINKS_MAX = 8;  // sinks per few-sink tile (mixed mode)
+// FP64 rows of tiles of one sink each: exact terms added in order (gravity_fp64.cu)
+int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st);
+// blocks of up to this many (sink, source) pairs go row by row, larger ones to gravity_cert.cu: a
+// row's latency is a few microseconds and its pairs cost five times as much.  Self-interacting
+// blocks of 400 / 1000 / 1500 / 2000 / 3000 bodies on GB300: rows 22 / 58 / 110 / 179 / 363 us,
+// gravity_cert.cu 60 / 98 / 140 / 169 / 228 us.
+constexpr int64_t FP64_ROW_PAIRS = 3200000;
 // mixed precision (gravity_mixed.cu): positions split into FP32 (hi, lo) once per evaluation
 struct SplitPos;
 constexpr int MIXED_SINKS_PER_TILE = 128;

@@ -29,6 +29,7 @@ UNITS = {
     "context.cu": ["-fmad=false"],
     "stages.cu": ["-fmad=false"],
     "gravity_fp64.cu": ["-fmad=false"],
+    "gravity_cert.cu": ["-fmad=false"],
     "gravity_mixed.cu": [],
     "ensemble.cu": ["-fmad=false"],
     "mlp.cu": [],

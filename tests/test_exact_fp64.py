@@ -90,3 +90,28 @@ def test_serial_sum_latency_on_the_gpu(tmp_path):
     serial, warp, _ = rows[0]
     assert warp < 0.6 * serial, r.stdout
     assert all(w < 2.0 * s_ for s_, w, _ in rows.values()), r.stdout
+
+
+def test_segmented_row_sum_on_the_cpu(tmp_path):
+    """warp_row_sum (csrc/row_sum.h) replayed lane by lane: the serial sum's bits on every row
+    family, the offset rules against chains added from shifted starts."""
+    exe = _build(tmp_path, "g++", "row_sum_check.cpp", ["-O2", "-std=c++17", "-ffp-contract=off"])
+    r = subprocess.run([exe, "8000"], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    terms, bad, rules, rbad = map(int, re.search(r"terms (\d+) bad (\d+) serial \d+ rules (\d+) rbad (\d+)",
+                                                 r.stdout).groups())
+    assert bad == 0 and rbad == 0 and terms > 6e7 and rules > 4e6
+    for fam in (0, 1):  # gravity-like and wide rows: hardly a lane added again
+        n, serial = map(int, re.search(rf"family {fam} terms (\d+) serial (\d+)", r.stdout).groups())
+        assert serial < 0.02 * n
+
+
+@pytest.mark.gpu
+def test_segmented_row_sum_on_the_gpu(tmp_path):
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    exe = _build(tmp_path, nvcc, "row_sum_gpu.cu",
+                 ["-gencode", "arch=compute_103a,code=sm_103a", "-O3", "-std=c++17", "-fmad=false"])
+    r = subprocess.run([exe, "20000"], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stdout + r.stderr
+    rows = re.findall(r"family (\d) rows (\d+) bad (\d+)", r.stdout)
+    assert len(rows) == 5 and all(int(bad) == 0 for _, _, bad in rows), r.stdout
