@@ -96,7 +96,10 @@ struct rg_ctx {
     double* d_records = nullptr;  // r and v as vec_t records (state in / out): 8 doubles per body
     double* d_astro = nullptr;    // astrocentric frame: per body the star's pull and indirect term (6 rows)
     int frame = RG_FRAME_BARY;    // pp_disk::frame_center
-    double* h_pin = nullptr;  // pinned: [0] dt, [1] max bits, [2..3] counts, [4..5] d_counters
+    double* h_pin = nullptr;  // pinned: [0] dt, [1] max bits, [2..3] counts, [4..5] d_counters, [8..] step_res
+    StepResult* step_res = nullptr;  // what a step kernel left for the host
+    bool counts_known = false;       // step_res holds the event counts of the step being collected
+    bool no_ejection = false;        // the last step's screen of the state as it is now found no candidate
     // host mirrors of the body parameters (authoritative; the state lives on the device)
     std::vector<rg_param_t> p;
     std::vector<rg_body_metadata_t> md;
@@ -281,6 +284,7 @@ void prof_end(rg_ctx* c, long idx)
 // --------------------------------------------------------------------- uploads / downloads
 int upload_params(rg_ctx* c)
 {
+    c->no_ejection = false;
     const int n = c->n_total();
     std::vector<double> m(n), R(n);
     std::vector<int> id(n), ty(n);
@@ -314,6 +318,7 @@ int download_state(rg_ctx* c, std::vector<double>& h)
 
 int upload_state(rg_ctx* c, const std::vector<double>& h)
 {
+    c->no_ejection = false;
     const int n = c->n_total();
     if (n > 0)
         RG_CUDA_CHECK(cudaMemcpy2DAsync(c->d_y, c->cap * sizeof(double), h.data(), n * sizeof(double),
@@ -335,6 +340,7 @@ int get_body(rg_ctx* c, int i, rg_vec_t* r, rg_vec_t* v)
 
 int set_body(rg_ctx* c, int i, const rg_vec_t& r, const rg_vec_t& v)
 {
+    c->no_ejection = false;
     const double h[6] = {r.x, r.y, r.z, v.x, v.y, v.z};
     RG_CUDA_CHECK(cudaMemcpy2DAsync(c->d_y + i, c->cap * sizeof(double), h, sizeof(double), sizeof(double), 6,
                                     cudaMemcpyHostToDevice, c->st));
@@ -344,6 +350,7 @@ int set_body(rg_ctx* c, int i, const rg_vec_t& r, const rg_vec_t& v)
 
 int set_param_dev(rg_ctx* c, int i)
 {
+    c->no_ejection = false;
     RG_CUDA_CHECK(cudaMemcpyAsync(c->d_mass + i, &c->p[i].mass, sizeof(double), cudaMemcpyHostToDevice, c->st));
     RG_CUDA_CHECK(cudaMemcpyAsync(c->d_radius + i, &c->p[i].radius, sizeof(double), cudaMemcpyHostToDevice, c->st));
     RG_CUDA_CHECK(cudaMemcpyAsync(c->d_id + i, &c->md[i].id, sizeof(int), cudaMemcpyHostToDevice, c->st));
@@ -364,6 +371,7 @@ enum {
 // light bodies per symmetric tile of one disk, about: one per thread of a 256-thread CTA up to
 // a wave of resident CTAs, so that a disk of a thousand bodies spreads over several SMs (the
 // evaluation's latency is one tile's)
+constexpr int FP64_ROWS_FEW = 128;   // row-kernel blocks (few sources) with at most this many sinks go a CTA per row
 constexpr int FEW_BLOCK_SINKS = 32;  // blocks with at most this many sinks use the few-sink path
 
 // CTA tiles of the interaction matrix (number_of_bodies::get_bound_SI/NSI/NI,
@@ -438,11 +446,14 @@ void build_tiles(rg_ctx* c)
             add_group(0, GROUP_PAIRPAR, b.s0, b.s1, b.src1, b.block, c->pairpar_S);
             continue;
         }
-        if (b.src1 <= c->rowseq_max_src) {  // few sources: thread per sink (same tiles in both modes)
+        // few sources: thread per sink, at 1.7 us per source -- a few sinks with more than a pair or
+        // two each are faster a CTA per row (nine bodies: 15.7 us against 4)
+        const bool rows = ns <= FP64_ROWS_FEW && b.src1 > 3;
+        if (b.src1 <= c->rowseq_max_src) {
             // tiles of up to 128 sinks; narrower ones when that leaves SMs idle (a thread's few
             // serial pair terms are latency-bound, so more SMs beat fuller CTAs)
             const int rs_step = ns >= 2 * 128 * c->n_sm ? 128 : (ns >= 2 * 64 * c->n_sm ? 64 : 32);
-            add_group(0, GROUP_ROWSEQ, b.s0, b.s1, b.src1, b.block, rs_step);
+            add_group(0, rows ? GROUP_FP64_ROWS : GROUP_ROWSEQ, b.s0, b.s1, b.src1, b.block, rows ? 1 : rs_step);
             if (sym && b.block == 1) {  // the heavy rows [0, nsi), then one segment per CTA (Tile::part from 1)
                 const size_t t0 = c->tiles.size();
                 std::vector<int> parts;
@@ -465,8 +476,7 @@ void build_tiles(rg_ctx* c)
                 }
                 c->plan[1].push_back(gr);
             } else {
-                c->plan[1].push_back(c->plan[0].back());
-                c->plan[1].back().kind = GROUP_DF_ROWSEQ;
+                add_group(1, GROUP_DF_ROWSEQ, b.s0, b.s1, b.src1, b.block, rs_step);
             }
             continue;
         }
@@ -818,10 +828,18 @@ int kernel_flag_error(rg_ctx* c, unsigned int flag)
 int collect_events(rg_ctx* c)
 {
     // the three counters in one copy to pinned memory: one round trip per step
-    unsigned int* const h_counts = reinterpret_cast<unsigned int*>(&c->h_pin[4]);
-    RG_CUDA_CHECK(cudaMemcpyAsync(h_counts, c->d_counters, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, c->st));
-    RG_CUDA_CHECK(cudaStreamSynchronize(c->st));
-    const unsigned int counts[3] = {h_counts[0], h_counts[1], h_counts[2]};
+    unsigned int counts[3];
+    if (c->counts_known) {
+        counts[0] = c->step_res->n_event;
+        counts[1] = c->step_res->n_hill;
+        counts[2] = 0u;
+        c->counts_known = false;
+    } else {
+        unsigned int* const h_counts = reinterpret_cast<unsigned int*>(&c->h_pin[4]);
+        RG_CUDA_CHECK(cudaMemcpyAsync(h_counts, c->d_counters, 3 * sizeof(unsigned int), cudaMemcpyDeviceToHost, c->st));
+        RG_CUDA_CHECK(cudaStreamSynchronize(c->st));
+        for (int k = 0; k < 3; k++) counts[k] = h_counts[k];
+    }
     if (int krc = kernel_flag_error(c, counts[2])) return krc;
     const int nsi = c->n_si();
     for (int kind = 0; kind < 2; kind++) {
@@ -1249,8 +1267,82 @@ bool replay_step_graph(rg_ctx* c, rg_ctx::StepGraph& sg, F body, int* rc)
     return true;
 }
 
+// A step of a small system: each attempt one kernel (small_step.cu), one synchronisation
+int step_rkf78_small(rg_ctx* c)
+{
+    SmallStepArgs a{};
+    a.g.mass = c->d_mass;
+    a.g.radius = c->d_radius;
+    a.g.id = c->d_id;
+    a.g.f_rad = c->thr[RG_THRESHOLD_RADII_ENHANCE_FACTOR];
+    a.g.hill_f3 = c->hill_factor * c->hill_factor * c->hill_factor;
+    a.g.record = (c->inner_steps && a.g.f_rad > 0.0) ? 1 : 0;
+    a.g.hill = c->hill_factor > 0.0 ? 1 : 0;
+    a.g.ev = EventBuf{c->d_ev, c->d_ev_count, c->ev_cap};
+    a.g.hv = EventBuf{c->d_hill, c->d_hill_count, c->ev_cap};
+    a.y = c->d_y;
+    a.y_out = c->d_yout;
+    a.k0 = c->d_k[0];
+    a.stride = c->cap;
+    a.n = c->n_total();
+    a.n_si = c->n_si();
+    a.n_massive = c->n_massive();
+    a.n_err = c->ectp ? a.n : a.n_massive;
+    a.adaptive = c->adaptive;
+    a.type = c->d_type;
+    a.thr_hit = c->thr[0];
+    a.thr_ej = c->thr[1];
+    a.thr_hit2 = c->thr[3];
+    a.thr_ej2 = c->thr[4];
+    for (int r = 1; r < 13; r++) {
+        a.nterm[r] = (signed char)rk8_nterm[r];
+        for (int q = 0; q < rk8_nterm[r]; q++) {
+            a.stage[r][q] = (signed char)rk8_stage[r][q];
+            a.a[r][q] = rk8_a[rk8_aidx[r][q]];
+        }
+    }
+    const double b[5] = {rk8_b[0], rk8_b[5], rk8_b[6], rk8_b[8], rk8_b[10]};
+    for (int q = 0; q < 5; q++) a.b[q] = b[q];
+    a.out = c->step_res;
+    double max_err = 0.0;
+    int iter = 0;
+    do {
+        c->dt_did = c->dt_try;
+        c->attempt_dt.push_back(c->dt_try);
+        a.dt = c->dt_try;
+        a.first = iter == 0;
+        a.attempt = (unsigned int)iter;
+        const int rc = launch_small_rkf78(a, c->st);
+        if (rc) return rc;
+        c->n_kernels++;
+        const int evals = c->r_max - 1 + (iter == 0);
+        c->n_gravity_evals += evals;
+        c->n_pairs += evals * c->pairs_per_eval;
+        RG_CUDA_CHECK(cudaStreamSynchronize(c->st));
+        if (c->adaptive) {
+            double raw;
+            std::memcpy(&raw, &c->step_res->max_bits, sizeof(raw));
+            max_err = std::fabs(c->dt_try * (41.0 / 840.0) * raw);
+            c->dt_try *= 0.9 * std::pow(c->tol / max_err, 1.0 / (c->order + 1));
+        }
+        iter++;
+    } while (c->adaptive && max_err > c->tol);
+    c->counts_known = true;
+    c->no_ejection = c->step_res->n_eject == 0;
+    update_counters(c, iter);
+    c->t += c->dt_did;
+    swap_y(c);
+    return RG_OK;
+}
+
 int step_rkf78(rg_ctx* c)
 {
+    // (up to SMALL_MAX bodies one SM is faster than a kernel per stage; timing hooks take the latter)
+    if (c->gravity_mode == RG_GRAVITY_FP64 && c->frame == RG_FRAME_BARY && c->n_total() <= SMALL_MAX && c->n_total() > 0 &&
+        !c->profiling && c->use_graphs) {
+        c->attempt_dt.clear();
+        return step_rkf78_small(c);
+    }
     const size_t cap = (size_t)c->cap;
     c->attempt_dt.clear();
     const int parity = c->d_y < c->d_yout ? 0 : 1;
@@ -1346,7 +1438,7 @@ int check_ejection_hit(rg_ctx* c, int* n_handled)
     if (n_handled) *n_handled = 0;
     const int n = c->n_total();
     const bool any = (0.0 < c->thr[RG_THRESHOLD_EJECTION_DISTANCE]) || (0.0 < c->thr[RG_THRESHOLD_HIT_CENTRUM_DISTANCE]);
-    if (any && n > 0) {
+    if (any && n > 0 && !c->no_ejection) {
         RG_CUDA_CHECK(cudaMemsetAsync(c->d_ej_count, 0, sizeof(unsigned int), c->st));
         int rc = launch_ejection(c->d_y, c->d_y + c->cap, c->d_y + 2 * (size_t)c->cap, c->d_id, c->d_type, n, c->thr,
                                  c->d_ej, c->d_ej_count, (unsigned int)c->cap, c->st);
@@ -1521,6 +1613,7 @@ int do_step(rg_ctx* c)
 {
     if (!c->has_int) return set_error(RG_ERR_STATE, "no integrator set (rg_set_integrator)");
     c->t_step = c->t;
+    c->no_ejection = c->counts_known = false;
     int rc;
     switch (c->int_type) {
     case RG_INT_EULER: rc = step_euler(c); break;
@@ -1656,8 +1749,9 @@ static int create_impl(const rg_counts_t* n, const rg_vec_t* r, const rg_vec_t* 
     chk(dalloc(&c->d_rf, nt));
     chk(dalloc(&c->d_smax, SCREEN_MAX_WORDS));
     chk(dalloc(&c->d_screen_slot, nt));
-    if (!rc && cudaMallocHost((void**)&c->h_pin, 8 * sizeof(double)) != cudaSuccess)
+    if (!rc && cudaMallocHost((void**)&c->h_pin, 16 * sizeof(double)) != cudaSuccess)
         chk(set_error(RG_ERR_NOMEM, "pinned host buffer"));
+    if (!rc) c->step_res = reinterpret_cast<StepResult*>(&c->h_pin[8]);
     if (frame == RG_FRAME_ASTRO) {
         chk(dalloc(&c->d_astro, (size_t)6 * nt));
         // the star's row of every derivative buffer is never written in this frame
@@ -1961,6 +2055,7 @@ int rg_get_state_internal(rg_ctx* c, rg_vec_t* r, rg_vec_t* v, rg_param_t* p, rg
 
 static int set_state_impl(rg_ctx* c, const rg_vec_t* r, const rg_vec_t* v)
 {
+    c->no_ejection = false;
     const int n = c->n_total();
     if (n > 0) {  // one copy per array, the rows built on the device (v / k as the host would)
         double* dr = c->d_records;

@@ -147,6 +147,29 @@ int launch_grav_df_sym(const GravArgs& g, const int* cta_seg, int n_cta, const v
 int launch_star_distance(const double* x, const double* y, const double* z, const int* base_of, int n, double* rho,
                          cudaStream_t st);
 
+// one attempt of an RKF7(8) step of at most SMALL_MAX bodies, FP64, barycentric (small_step.cu)
+constexpr int SMALL_MAX = 32;
+struct StepResult {  // in pinned host memory
+    unsigned long long max_bits;
+    unsigned int n_event, n_hill, n_eject;  // n_eject: candidates of the ejection / hit-star screen of y_out
+};
+struct SmallStepArgs {
+    GravArgs g;  // mass, radius, id, event options and buffers
+    const double* y;
+    double* y_out;
+    double* k0;     // the step's first stage vector: written by its first attempt, read by the others
+    int stride, n, n_si, n_massive, n_err;
+    int first, adaptive;
+    unsigned int attempt;
+    double dt;
+    const int* type;
+    double thr_hit, thr_ej, thr_hit2, thr_ej2;
+    double a[13][MAXT], b[5];
+    signed char nterm[13], stage[13][MAXT];
+    StepResult* out;
+};
+int launch_small_rkf78(const SmallStepArgs& a, cudaStream_t st);
+
 int measure_pipe_peak(int kind, double* tflops);
 
 }  // namespace redgb

@@ -30,6 +30,7 @@ UNITS = {
     "stages.cu": ["-fmad=false"],
     "gravity_fp64.cu": ["-fmad=false"],
     "gravity_cert.cu": ["-fmad=false"],
+    "small_step.cu": ["-fmad=false"],
     "gravity_mixed.cu": [],
     "ensemble.cu": ["-fmad=false"],
     "mlp.cu": [],
