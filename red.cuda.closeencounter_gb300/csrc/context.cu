@@ -734,14 +734,13 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
                 c->n_kernels++;
             }
             if (!rc) {
-                // split the sources over grid.y so that about 4 CTAs per SM are in flight
                 const int src = c->tiles[gr.off].src_end - c->tiles[gr.off].src_begin;
                 const int src_tiles = (src + MIXED_SOURCE_TILE - 1) / MIXED_SOURCE_TILE;
                 int chunk;
                 if (c->mixed_chunk_src > 0) {
                     chunk = std::min(c->mixed_chunk_src, src_tiles * MIXED_SOURCE_TILE);
                 } else {
-                    const int n = std::max(1, std::min((4 * c->n_sm + gr.n - 1) / gr.n, src / (4 * MIXED_SOURCE_TILE)));
+                    const int n = mixed_chunk_count(gr.n, src_tiles, c->n_sm);
                     chunk = (src_tiles + n - 1) / n * MIXED_SOURCE_TILE;
                 }
                 const int chunks = (src + chunk - 1) / chunk;

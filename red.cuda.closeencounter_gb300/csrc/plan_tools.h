@@ -8,6 +8,21 @@
 
 namespace redgb {
 
+// Source chunks (grid.y) of the mixed tile kernel, two CTAs to an SM, for `sink_tiles` tiles of
+// sinks and `src_tiles` tiles of sources: as many as fit in one wave of CTAs, or, where that
+// leaves fewer, enough for 16 waves in chunks of at least six source tiles (a CTA starts with its
+// sinks and the heavy sources, so shorter chunks repeat more of that; a grid of one to three
+// waves leaves the chip to the last of them).  Evaluations on GB300, one chunk per about 4 CTAs
+// an SM -> this rule: 1001 bodies 43.7 -> 28 us, 3001 60.5 -> 36 us, 16 385 358 -> 319 us,
+// 131 074 16.56 -> 15.7 ms.
+inline int mixed_chunk_count(int sink_tiles, int src_tiles, int n_sm)
+{
+    const int64_t slots = 2 * (int64_t)std::max(n_sm, 1), tiles = std::max(sink_tiles, 1);
+    const int64_t one_wave = slots / tiles;
+    const int64_t many = std::min<int64_t>((16 * slots + tiles - 1) / tiles, src_tiles / 6);
+    return (int)std::max<int64_t>(1, std::min<int64_t>(std::max(one_wave, many), src_tiles));
+}
+
 // Segments of the symmetric heavy-light kernel (grav_df_sym).  `systems` holds one tile per
 // system: its light bodies [sink_begin, sink_end) (and whatever else the kernel reads, copied
 // into every segment).  The kernel's CTA takes a segment in passes of `unit` bodies (one per
