@@ -7,21 +7,23 @@
 //
 // Parameter vector (FP32 master copy; the forward passes read its BF16 image):
 //   W1[64][8] b1[64] W2[64][64] b2[64] w3[64] b3
-// Training: a CTA owns a tile of MLP_TB samples; activations live in shared memory, the
-// matrix products are plain FP32 FMA loops (the network has 4.8k weights -- far too small
-// for the tensor cores to matter), and each CTA adds its partial gradient to a global FP32
-// buffer with atomics.
+// Training: CTAs walk tiles of MLP_TB samples with the activations in shared memory; the
+// matrix products are register-tiled FP32 FMA loops (the activations and their gradients stay
+// FP32, which the tensor cores do not take), the weight gradients stay in registers from tile
+// to tile, and each CTA adds its sums to a global FP32 buffer once, with atomics.
 #include <cuda_bf16.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <random>
 #include <string>
 #include <vector>
 
 #include "../../include/redgb.h"
+#include "abi_guard.h"
 #include "common.cuh"
 #include "mlp.h"
 
@@ -44,114 +46,277 @@ __global__ void mlp_to_bf16(const float* __restrict__ w, __nv_bfloat16* __restri
 
 __device__ __forceinline__ float bf(const __nv_bfloat16* w, int i) { return __bfloat162float(w[i]); }
 
-// Forward (and optionally backward) of a tile of samples.  x: n x 8 (already
-// standardised), y: targets (training) ; out: predictions; grad: += dL/dw (FP32).
+struct MlpNorm {
+    float mean[MLP_IN], std[MLP_IN];
+};
+
+// Shared-memory matrices are H rows of MLP_TB or H columns, padded so that a row starts four
+// banks after the one before it: the float4 stores of 8 neighbouring lanes to 8 neighbouring
+// rows touch every bank once.  A thread's four units are u = (t & 15) + 16 j; in rows over
+// units they stand together (position 4 (u & 15) + (u >> 4)), one float4.
+constexpr int MLP_PITCH = MLP_TB + 4;
+constexpr int MLP_MAT = MLP_HIDDEN * MLP_PITCH;
+static_assert(MLP_TB == MLP_HIDDEN && MLP_TB == 64, "256 threads hold a tile as 4 x 4 blocks");
+__device__ __forceinline__ int mlp_pos(int u) { return ((u & 15) << 2) | (u >> 4); }
+
+struct MlpSmem {
+    float W1t[MLP_IN][MLP_HIDDEN];  // [f][position of u]
+    float X[MLP_TB][MLP_IN];        // standardised inputs
+    float b1[MLP_HIDDEN], b2[MLP_HIDDEN], w3[MLP_HIDDEN];
+    float D[MLP_TB];  // dL/dy per sample
+    float W2t[MLP_MAT];  // [v][position of u]
+    float A1t[MLP_MAT];  // silu(Z1), [v][s]
+    float A2t[MLP_MAT];  // silu(Z2), [u][s]; then dL/dZ2, [u][s]
+};
+struct MlpTrainSmem : MlpSmem {
+    float W2p[MLP_MAT];  // [u][position of v]
+    float A1p[MLP_MAT];  // silu(Z1), [s][position of v]
+    float G2p[MLP_MAT];  // dL/dZ2, [s][position of u]
+};
+// The loss of a batch: 32 samples are added before they go to the sum.  Above this many samples
+// each goes there by itself: the rounding of that long a serial sum (2.5e-5 of the loss at
+// 100 000 samples, against 1e-7) is in every loss that callers have kept of such batches, and
+// those stay comparable.  It is what bounds such a batch: 1.9 ns an addition to one address.
+constexpr int MLP_SERIAL_LOSS = 65536;
+constexpr int MLP_FORWARD_CTAS = 3;  // per SM (training: 2)
+constexpr int MLP_GROUP = MLP_HIDDEN * (MLP_IN + 1);  // dW1 and db1 of one sample group
+static_assert(16 * MLP_GROUP <= 3 * MLP_MAT, "the groups' sums fit over the last three matrices");
+static_assert(sizeof(MlpSmem) % 16 == 0, "float4 rows");
+
+// acc[i][j] += sum over k of A[k][4 a + i] B[k][4 b + j], k ascending
+__device__ __forceinline__ void mlp_mma(float (&acc)[4][4], const float* A, const float* B)
+{
+#pragma unroll 8
+    for (int k = 0; k < 64; k++) {
+        const float4 a = *reinterpret_cast<const float4*>(A + k * MLP_PITCH);
+        const float4 b = *reinterpret_cast<const float4*>(B + k * MLP_PITCH);
+        const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+    }
+}
+
+// Forward (and optionally backward) of the samples.  x: n x 8; y: targets (training); index:
+// the samples' rows or null; out: predictions; grad: += dL/dw and, behind it, += the loss (FP32).
+// Thread t holds samples 4 (t / 16) .. + 3 and units (t & 15) + 16 j of a tile of 64.
+// Bound: the FP32 pipe (three 64 x 64 x 64 products a tile in training, one in the forward
+// pass) behind the SiLUs and the barriers between the phases; 16 warps an SM in training, limited
+// by the matrices' shared memory, 24 in the forward pass (16: 55 us, 32: as 24).  A thread's 4 x 4
+// block reads two float4 for 16 FMAs, each SiLU is taken once, and the weights' gradients go to
+// global memory once a CTA; one output per thread with its operands and SiLUs from shared memory
+// and a CTA's atomics per 32 samples took 280 us (forward) and 617 us (training) for 100 000
+// samples, this 46 and 190 us.
 template <bool TRAIN>
-__global__ void __launch_bounds__(256) mlp_tile_kernel(const __nv_bfloat16* __restrict__ wb, const float* __restrict__ x,
-                                                      const float* __restrict__ y, const int* __restrict__ index, int n,
-                                                      float inv_batch, float* __restrict__ out,
-                                                      float* __restrict__ grad, float* __restrict__ loss)
+__global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
+    mlp_tile_kernel(const __nv_bfloat16* __restrict__ wb, const MlpNorm norm, const float* __restrict__ x,
+                    const float* __restrict__ y, const int* __restrict__ index, int n, float inv_batch,
+                    float* __restrict__ out, float* __restrict__ grad)
 {
     constexpr int H = MLP_HIDDEN, I = MLP_IN, TB = MLP_TB;
-    __shared__ float X[TB][I];
-    __shared__ float Z1[TB][H + 1];
-    __shared__ float Z2[TB][H + 1];
-    __shared__ float D[TB];   // dL/dy per sample
-    __shared__ float W2s[H][H + 1];
-    const int t = threadIdx.x;
-    const int s0 = blockIdx.x * TB;
-    for (int k = t; k < TB * I; k += blockDim.x) {
-        const int s = k / I, f = k % I;
-        const int g = s0 + s;
-        X[s][f] = g < n ? x[(size_t)(index ? index[g] : g) * I + f] : 0.0f;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    MlpTrainSmem& S = *reinterpret_cast<MlpTrainSmem*>(smem_raw);  // the forward pass stops at MlpSmem's end
+    const int t = threadIdx.x, ug = t & 15, sg = t >> 4, s0 = 4 * sg;
+    for (int k = t; k < H * I; k += 256) S.W1t[k % I][mlp_pos(k / I)] = bf(wb, MLP_OFF_W1 + k);
+    for (int k = t; k < H * H; k += 256) {
+        const float w = bf(wb, MLP_OFF_W2 + k);
+        S.W2t[(k % H) * MLP_PITCH + mlp_pos(k / H)] = w;
+        if (TRAIN) S.W2p[(k / H) * MLP_PITCH + mlp_pos(k % H)] = w;
     }
-    for (int k = t; k < H * H; k += blockDim.x) W2s[k / H][k % H] = bf(wb, MLP_OFF_W2 + k);
-    __syncthreads();
-    // layer 1: Z1 = X W1^T + b1
-    for (int k = t; k < TB * H; k += blockDim.x) {
-        const int s = k / H, u = k % H;
-        float z = bf(wb, MLP_OFF_B1 + u);
+    if (t < H) {
+        S.b1[t] = bf(wb, MLP_OFF_B1 + t);
+        S.b2[t] = bf(wb, MLP_OFF_B2 + t);
+        S.w3[t] = bf(wb, MLP_OFF_W3 + t);
+    }
+    const float b3 = bf(wb, MLP_OFF_B3);
+    [[maybe_unused]] float gw2[4][4], gw1[4][I], gb1[4], gw3 = 0.0f, gb2 = 0.0f, gb3 = 0.0f;
 #pragma unroll
-        for (int f = 0; f < I; f++) z = fmaf(bf(wb, MLP_OFF_W1 + u * I + f), X[s][f], z);
-        Z1[s][u] = z;
+    for (int j = 0; j < 4; j++) {
+        gb1[j] = 0.0f;
+#pragma unroll
+        for (int i = 0; i < 4; i++) gw2[i][j] = 0.0f;
+#pragma unroll
+        for (int f = 0; f < I; f++) gw1[j][f] = 0.0f;
     }
-    __syncthreads();
-    // layer 2: Z2 = silu(Z1) W2^T + b2
-    for (int k = t; k < TB * H; k += blockDim.x) {
-        const int s = k / H, u = k % H;
-        float z = bf(wb, MLP_OFF_B2 + u);
-        for (int v = 0; v < H; v++) z = fmaf(W2s[u][v], silu(Z1[s][v]), z);
-        Z2[s][u] = z;
-    }
-    __syncthreads();
-    // output: y = w3 . silu(Z2) + b3
-    for (int s = t; s < TB; s += blockDim.x) {
-        float o = bf(wb, MLP_OFF_B3);
-        for (int u = 0; u < H; u++) o = fmaf(bf(wb, MLP_OFF_W3 + u), silu(Z2[s][u]), o);
-        const int g = s0 + s;
-        if (g < n) {
-            if (out) out[g] = o;
-            if (TRAIN) {
-                const float r = o - y[index ? index[g] : g];
-                D[s] = 2.0f * r * inv_batch;
-                atomicAdd(loss, r * r * inv_batch);
+    const int tiles = n / TB + (n % TB != 0);
+    for (int tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int first = tile * TB, ns = min(TB, n - first);
+        if (t < 2 * TB) {  // four inputs of sample t / 2
+            const int s = t >> 1, f = 4 * (t & 1);
+            float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (s < ns) {
+                v = *reinterpret_cast<const float4*>(x + (size_t)(index ? index[first + s] : first + s) * I + f);
+                v.x = __fdiv_rn(v.x - norm.mean[f], norm.std[f]);
+                v.y = __fdiv_rn(v.y - norm.mean[f + 1], norm.std[f + 1]);
+                v.z = __fdiv_rn(v.z - norm.mean[f + 2], norm.std[f + 2]);
+                v.w = __fdiv_rn(v.w - norm.mean[f + 3], norm.std[f + 3]);
             }
-        } else {
-            D[s] = 0.0f;
+            *reinterpret_cast<float4*>(&S.X[s][f]) = v;
+        }
+        __syncthreads();
+        [[maybe_unused]] float ds1[4][4];
+        float acc[4][4];
+        // layer 1: Z1 = X W1^T + b1
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float b = S.b1[ug + 16 * j];
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i][j] = b;
+        }
+#pragma unroll
+        for (int f = 0; f < I; f++) {
+            const float4 w = *reinterpret_cast<const float4*>(&S.W1t[f][4 * ug]);
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float v = S.X[s0 + i][f];
+                acc[i][0] = fmaf(w.x, v, acc[i][0]);
+                acc[i][1] = fmaf(w.y, v, acc[i][1]);
+                acc[i][2] = fmaf(w.z, v, acc[i][2]);
+                acc[i][3] = fmaf(w.w, v, acc[i][3]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                if (TRAIN) ds1[i][j] = dsilu(acc[i][j]);
+                acc[i][j] = silu(acc[i][j]);
+            }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<float4*>(&S.A1t[(ug + 16 * j) * MLP_PITCH + s0]) =
+                make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+        if constexpr (TRAIN)
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<float4*>(&S.A1p[(s0 + i) * MLP_PITCH + 4 * ug]) =
+                    make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        __syncthreads();
+        // layer 2: Z2 = silu(Z1) W2^T + b2
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float b = S.b2[ug + 16 * j];
+#pragma unroll
+            for (int i = 0; i < 4; i++) acc[i][j] = b;
+        }
+        mlp_mma(acc, S.A1t + s0, S.W2t + 4 * ug);
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            *reinterpret_cast<float4*>(&S.A2t[(ug + 16 * j) * MLP_PITCH + s0]) =
+                make_float4(silu(acc[0][j]), silu(acc[1][j]), silu(acc[2][j]), silu(acc[3][j]));
+        __syncthreads();
+        // output: y = w3 . silu(Z2) + b3
+        if (t < TB) {
+            float o = b3;
+#pragma unroll 16
+            for (int u = 0; u < H; u++) o = fmaf(S.w3[u], S.A2t[u * MLP_PITCH + t], o);
+            [[maybe_unused]] float d = 0.0f, e = 0.0f;
+            if (t < ns) {
+                if (out) out[first + t] = o;
+                if (TRAIN) {
+                    const float r = o - y[index ? index[first + t] : first + t];
+                    d = 2.0f * r * inv_batch;
+                    e = r * r * inv_batch;
+                }
+            }
+            if constexpr (TRAIN) {
+                S.D[t] = d;
+                gb3 += d;
+                if (n > MLP_SERIAL_LOSS) {
+                    if (t < ns) atomicAdd(&grad[MLP_NPARAM], e);
+                } else {
+                    for (int q = 1; q < 32; q <<= 1) e += __shfl_xor_sync(0xffffffffu, e, q);
+                    if ((t & 31) == 0) atomicAdd(&grad[MLP_NPARAM], e);
+                }
+            }
+        }
+        __syncthreads();
+        if constexpr (TRAIN) {
+            // backward.  dw3 = sum_s D_s silu(Z2_s): unit t / 4, a quarter of the samples
+            {
+                const float* a = &S.A2t[(t >> 2) * MLP_PITCH + 16 * (t & 3)];
+#pragma unroll
+                for (int q = 0; q < 16; q++) gw3 = fmaf(S.D[16 * (t & 3) + q], a[q], gw3);
+            }
+            __syncthreads();
+            // dZ2 = D w3 silu'(Z2)
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float w = S.w3[ug + 16 * j];
+#pragma unroll
+                for (int i = 0; i < 4; i++) acc[i][j] = S.D[s0 + i] * w * dsilu(acc[i][j]);
+                *reinterpret_cast<float4*>(&S.A2t[(ug + 16 * j) * MLP_PITCH + s0]) =
+                    make_float4(acc[0][j], acc[1][j], acc[2][j], acc[3][j]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+                *reinterpret_cast<float4*>(&S.G2p[(s0 + i) * MLP_PITCH + 4 * ug]) =
+                    make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+            __syncthreads();
+            // db2[u] = sum_s dZ2[s][u]
+            {
+                const float* a = &S.A2t[(t >> 2) * MLP_PITCH + 16 * (t & 3)];
+#pragma unroll
+                for (int q = 0; q < 16; q++) gb2 += a[q];
+            }
+            // dW2[u][v] = sum_s dZ2[s][u] silu(Z1[s][v]): units sg + 16 i
+            mlp_mma(gw2, S.G2p + 4 * sg, S.A1p + 4 * ug);
+            // dZ1[s][v] = (sum_u dZ2[s][u] W2[u][v]) silu'(Z1[s][v])
+#pragma unroll
+            for (int i = 0; i < 4; i++)
+#pragma unroll
+                for (int j = 0; j < 4; j++) acc[i][j] = 0.0f;
+            mlp_mma(acc, S.A2t + s0, S.W2p + 4 * ug);
+            // dW1[v][f] = sum_s dZ1[s][v] X[s][f]; db1[v] = sum_s dZ1[s][v]
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const float4 xa = *reinterpret_cast<const float4*>(&S.X[s0 + i][0]);
+                const float4 xb = *reinterpret_cast<const float4*>(&S.X[s0 + i][4]);
+                const float xv[8] = {xa.x, xa.y, xa.z, xa.w, xb.x, xb.y, xb.z, xb.w};
+#pragma unroll
+                for (int j = 0; j < 4; j++) {
+                    const float d = acc[i][j] * ds1[i][j];
+                    gb1[j] += d;
+#pragma unroll
+                    for (int f = 0; f < I; f++) gw1[j][f] = fmaf(d, xv[f], gw1[j][f]);
+                }
+            }
+            __syncthreads();  // the next tile overwrites X and the matrices
         }
     }
-    if (!TRAIN) return;
-    __syncthreads();
-    // backward.  dw3 = sum_s D_s silu(Z2_s); db3 = sum_s D_s
-    for (int u = t; u < H; u += blockDim.x) {
-        float g3 = 0.0f;
-        for (int s = 0; s < TB; s++) g3 = fmaf(D[s], silu(Z2[s][u]), g3);
-        atomicAdd(&grad[MLP_OFF_W3 + u], g3);
+    if constexpr (!TRAIN) return;
+    // the CTA's sums, once
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) atomicAdd(&grad[MLP_OFF_W2 + (sg + 16 * i) * H + ug + 16 * j], gw2[i][j]);
+    float* const g = S.W2p + sg * MLP_GROUP;
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+#pragma unroll
+        for (int f = 0; f < I; f++) g[(ug + 16 * j) * (I + 1) + f] = gw1[j][f];
+        g[(ug + 16 * j) * (I + 1) + I] = gb1[j];
     }
-    if (t == 0) {
-        float gb = 0.0f;
-        for (int s = 0; s < TB; s++) gb += D[s];
-        atomicAdd(&grad[MLP_OFF_B3], gb);
+    for (int d = 1; d < 4; d <<= 1) {
+        gw3 += __shfl_xor_sync(0xffffffffu, gw3, d);
+        gb2 += __shfl_xor_sync(0xffffffffu, gb2, d);
     }
-    __syncthreads();
-    // dZ2 = D w3 * silu'(Z2)  (overwrite Z2 with dZ2 after keeping silu(Z1) available)
-    for (int k = t; k < TB * H; k += blockDim.x) {
-        const int s = k / H, u = k % H;
-        Z2[s][u] = D[s] * bf(wb, MLP_OFF_W3 + u) * dsilu(Z2[s][u]);
+    if ((t & 3) == 0) {
+        atomicAdd(&grad[MLP_OFF_W3 + (t >> 2)], gw3);
+        atomicAdd(&grad[MLP_OFF_B2 + (t >> 2)], gb2);
     }
-    __syncthreads();
-    // dW2[u][v] = sum_s dZ2[s][u] silu(Z1[s][v]); db2[u] = sum_s dZ2[s][u]
-    for (int k = t; k < H * H; k += blockDim.x) {
-        const int u = k / H, v = k % H;
-        float g = 0.0f;
-        for (int s = 0; s < TB; s++) g = fmaf(Z2[s][u], silu(Z1[s][v]), g);
-        atomicAdd(&grad[MLP_OFF_W2 + k], g);
-    }
-    for (int u = t; u < H; u += blockDim.x) {
-        float g = 0.0f;
-        for (int s = 0; s < TB; s++) g += Z2[s][u];
-        atomicAdd(&grad[MLP_OFF_B2 + u], g);
+    if (t < TB) {
+        for (int d = 1; d < 32; d <<= 1) gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
+        if ((t & 31) == 0) atomicAdd(&grad[MLP_OFF_B3], gb3);
     }
     __syncthreads();
-    // dZ1[s][v] = (sum_u dZ2[s][u] W2[u][v]) silu'(Z1[s][v])  (into Z1)
-    for (int k = t; k < TB * H; k += blockDim.x) {
-        const int s = k / H, v = k % H;
-        float d = 0.0f;
-        for (int u = 0; u < H; u++) d = fmaf(Z2[s][u], W2s[u][v], d);
-        Z1[s][v] = d * dsilu(Z1[s][v]);
-    }
-    __syncthreads();
-    // dW1[u][f] = sum_s dZ1[s][u] X[s][f]; db1[u] = sum_s dZ1[s][u]
-    for (int k = t; k < H * I; k += blockDim.x) {
-        const int u = k / I, f = k % I;
-        float g = 0.0f;
-        for (int s = 0; s < TB; s++) g = fmaf(Z1[s][u], X[s][f], g);
-        atomicAdd(&grad[MLP_OFF_W1 + k], g);
-    }
-    for (int u = t; u < H; u += blockDim.x) {
-        float g = 0.0f;
-        for (int s = 0; s < TB; s++) g += Z1[s][u];
-        atomicAdd(&grad[MLP_OFF_B1 + u], g);
+    for (int k = t; k < MLP_GROUP; k += 256) {
+        float v = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 16; q++) v += S.W2p[q * MLP_GROUP + k];
+        const int u = k / (I + 1), f = k % (I + 1);
+        atomicAdd(&grad[f < I ? MLP_OFF_W1 + u * I + f : MLP_OFF_B1 + u], v);
     }
 }
 
@@ -184,9 +349,16 @@ struct rg_mlp {
     float* d_w = nullptr;
     float* d_m = nullptr;
     float* d_v = nullptr;
-    float* d_g = nullptr;
+    float* d_g = nullptr;  // gradient and, behind it, the loss
     __nv_bfloat16* d_wb = nullptr;
-    float* d_loss = nullptr;
+    float* h_g = nullptr;  // pinned copy of d_g
+    // samples of the last calls (grown, freed with the network): a call holds `lock` while it
+    // uses them and the gradient buffer
+    float *d_x = nullptr, *d_y = nullptr;
+    int* d_idx = nullptr;
+    size_t cap_x = 0, cap_y = 0, cap_idx = 0;
+    int n_sm = 0;
+    std::mutex lock;
     int64_t step = 0;
     cudaStream_t st = nullptr;
 };
@@ -236,9 +408,22 @@ int create_impl(uint64_t seed, rg_mlp** out)
     if (!rc) rc = dalloc(&m->d_w, MLP_NPARAM);
     if (!rc) rc = dalloc(&m->d_m, MLP_NPARAM);
     if (!rc) rc = dalloc(&m->d_v, MLP_NPARAM);
-    if (!rc) rc = dalloc(&m->d_g, MLP_NPARAM);
+    if (!rc) rc = dalloc(&m->d_g, MLP_NPARAM + 1);
     if (!rc) rc = dalloc(&m->d_wb, MLP_NPARAM);
-    if (!rc) rc = dalloc(&m->d_loss, 1);
+    if (!rc && cudaMallocHost((void**)&m->h_g, (MLP_NPARAM + 1) * sizeof(float)) != cudaSuccess) {
+        m->h_g = nullptr;
+        cudaGetLastError();
+        rc = set_error(RG_ERR_NOMEM, "cudaMallocHost (mlp)");
+    }
+    int dev = 0;
+    if (!rc && (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&m->n_sm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess))
+        rc = set_error(RG_ERR_CUDA, "device attributes");
+    if (!rc && (cudaFuncSetAttribute(mlp_tile_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(MlpSmem)) != cudaSuccess ||
+                cudaFuncSetAttribute(mlp_tile_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)sizeof(MlpTrainSmem)) != cudaSuccess))
+        rc = set_error(RG_ERR_CUDA, "shared memory of the proposer's kernels");
     if (!rc && cudaMemcpy(m->d_w, m->w.data(), MLP_NPARAM * sizeof(float), cudaMemcpyHostToDevice) != cudaSuccess)
         rc = set_error(RG_ERR_CUDA, "upload");
     if (!rc && cudaMemset(m->d_m, 0, MLP_NPARAM * sizeof(float)) != cudaSuccess) rc = RG_ERR_CUDA;
@@ -253,29 +438,112 @@ int create_impl(uint64_t seed, rg_mlp** out)
     return RG_OK;
 }
 
-// standardised copy of the inputs
-std::vector<float> standardise(const rg_mlp* m, const float* x, int n)
+template <class T>
+int reserve(T** p, size_t* cap, size_t n)
 {
-    std::vector<float> z((size_t)n * MLP_IN);
-    for (int s = 0; s < n; s++)
-        for (int f = 0; f < MLP_IN; f++)
-            z[(size_t)s * MLP_IN + f] = (x[(size_t)s * MLP_IN + f] - m->norm_mean[f]) / m->norm_std[f];
-    return z;
+    if (n <= *cap) return RG_OK;
+    cudaFree(*p);
+    *p = nullptr;
+    *cap = 0;
+    const int rc = dalloc(p, n);
+    if (!rc) *cap = n;
+    return rc;
+}
+
+// the inputs (and targets) in the network's device buffers
+int upload(rg_mlp* m, const float* x, const float* y, int n)
+{
+    int rc = reserve(&m->d_x, &m->cap_x, (size_t)n * MLP_IN);
+    if (!rc) rc = reserve(&m->d_y, &m->cap_y, (size_t)n);
+    if (!rc)
+        RG_CUDA_CHECK(cudaMemcpyAsync(m->d_x, x, (size_t)n * MLP_IN * sizeof(float), cudaMemcpyHostToDevice, m->st));
+    if (!rc && y) RG_CUDA_CHECK(cudaMemcpyAsync(m->d_y, y, n * sizeof(float), cudaMemcpyHostToDevice, m->st));
+    return rc;
 }
 
 int run_tiles(rg_mlp* m, bool train, const float* d_x, const float* d_y, const int* d_idx, int n, float* d_out,
               float inv_batch)
 {
-    const int grid = (n + MLP_TB - 1) / MLP_TB;
-    if (grid <= 0) return RG_OK;
+    if (n <= 0) return RG_OK;
+    const int grid = std::min(n / MLP_TB + (n % MLP_TB != 0), (train ? 2 : MLP_FORWARD_CTAS) * m->n_sm);
+    MlpNorm norm;
+    for (int f = 0; f < MLP_IN; f++) {
+        norm.mean[f] = m->norm_mean[f];
+        norm.std[f] = m->norm_std[f];
+    }
     if (train)
-        mlp_tile_kernel<true><<<grid, 256, 0, m->st>>>(m->d_wb, d_x, d_y, d_idx, n, inv_batch, d_out, m->d_g,
-                                                       m->d_loss);
+        mlp_tile_kernel<true><<<grid, 256, sizeof(MlpTrainSmem), m->st>>>(m->d_wb, norm, d_x, d_y, d_idx, n, inv_batch,
+                                                                          d_out, m->d_g);
     else
-        mlp_tile_kernel<false><<<grid, 256, 0, m->st>>>(m->d_wb, d_x, d_y, d_idx, n, inv_batch, d_out, nullptr,
-                                                        nullptr);
+        mlp_tile_kernel<false><<<grid, 256, sizeof(MlpSmem), m->st>>>(m->d_wb, norm, d_x, d_y, d_idx, n, inv_batch,
+                                                                      d_out, nullptr);
     RG_CUDA_CHECK(cudaGetLastError());
     return RG_OK;
+}
+
+int zero_gradient(rg_mlp* m)
+{
+    RG_CUDA_CHECK(cudaMemsetAsync(m->d_g, 0, (MLP_NPARAM + 1) * sizeof(float), m->st));
+    return RG_OK;
+}
+
+int forward_impl(rg_mlp* m, const float* x, int n, float* y)
+{
+    std::lock_guard<std::mutex> hold(m->lock);
+    int rc = upload(m, x, nullptr, n);
+    if (!rc) rc = run_tiles(m, false, m->d_x, nullptr, nullptr, n, m->d_y, 0.0f);
+    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(y, m->d_y, n * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
+    return rc;
+}
+
+int gradient_impl(rg_mlp* m, const float* x, const float* y, int n, float* grads, float* loss)
+{
+    std::lock_guard<std::mutex> hold(m->lock);
+    int rc = upload(m, x, y, n);
+    if (!rc) rc = zero_gradient(m);
+    if (!rc) rc = run_tiles(m, true, m->d_x, m->d_y, nullptr, n, nullptr, 1.0f / (float)n);
+    if (!rc)
+        RG_CUDA_CHECK(cudaMemcpyAsync(m->h_g, m->d_g, (MLP_NPARAM + 1) * sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
+    if (rc) return rc;
+    std::memcpy(grads, m->h_g, MLP_NPARAM * sizeof(float));
+    if (loss) *loss = m->h_g[MLP_NPARAM];
+    return RG_OK;
+}
+
+int train_impl(rg_mlp* m, const float* x, const float* y, int n, int epochs, int batch, float lr, float weight_decay,
+               uint64_t seed, float* final_loss)
+{
+    std::lock_guard<std::mutex> hold(m->lock);
+    int rc = upload(m, x, y, n);
+    if (!rc) rc = reserve(&m->d_idx, &m->cap_idx, (size_t)n);
+    if (rc) return rc;
+    std::vector<int> idx(n);
+    for (int i = 0; i < n; i++) idx[i] = i;
+    std::mt19937_64 rng(seed);
+    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+    for (int ep = 0; ep < epochs && !rc; ep++) {
+        std::shuffle(idx.begin(), idx.end(), rng);
+        RG_CUDA_CHECK(cudaMemcpyAsync(m->d_idx, idx.data(), n * sizeof(int), cudaMemcpyHostToDevice, m->st));
+        for (int b0 = 0; b0 < n && !rc; b0 += batch) {
+            const int nb = std::min(batch, n - b0);
+            rc = zero_gradient(m);
+            if (!rc) rc = run_tiles(m, true, m->d_x, m->d_y, m->d_idx + b0, nb, nullptr, 1.0f / (float)nb);
+            if (rc) break;
+            m->step++;
+            const float bc1 = 1.0f - std::pow(b1, (float)m->step), bc2 = 1.0f - std::pow(b2, (float)m->step);
+            mlp_adamw_kernel<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->d_w, m->d_m, m->d_v, m->d_g, MLP_NPARAM, lr,
+                                                                        b1, b2, eps, weight_decay, bc1, bc2);
+            RG_CUDA_CHECK(cudaGetLastError());
+            rc = sync_bf16(m);
+        }
+    }
+    if (!rc)
+        RG_CUDA_CHECK(cudaMemcpyAsync(m->h_g, m->d_g + MLP_NPARAM, sizeof(float), cudaMemcpyDeviceToHost, m->st));
+    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
+    if (!rc && final_loss) *final_loss = m->h_g[0];
+    return rc;
 }
 
 }  // namespace
@@ -301,7 +569,10 @@ int rg_mlp_destroy(rg_mlp* m)
     cudaFree(m->d_v);
     cudaFree(m->d_g);
     cudaFree(m->d_wb);
-    cudaFree(m->d_loss);
+    cudaFree(m->d_x);
+    cudaFree(m->d_y);
+    cudaFree(m->d_idx);
+    cudaFreeHost(m->h_g);
     if (m->st) cudaStreamDestroy(m->st);
     delete m;
     return RG_OK;
@@ -348,40 +619,14 @@ int rg_mlp_forward(rg_mlp* m, const float* x, int n, float* y)
 {
     if (!m || n < 0 || (n > 0 && (!x || !y))) return set_error(RG_ERR_ARG, "bad argument");
     if (n == 0) return RG_OK;
-    std::vector<float> z = standardise(m, x, n);
-    float *d_x = nullptr, *d_o = nullptr;
-    int rc = dalloc(&d_x, z.size());
-    if (!rc) rc = dalloc(&d_o, (size_t)n);
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(d_x, z.data(), z.size() * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    if (!rc) rc = run_tiles(m, false, d_x, nullptr, nullptr, n, d_o, 0.0f);
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(y, d_o, n * sizeof(float), cudaMemcpyDeviceToHost, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
-    cudaFree(d_x);
-    cudaFree(d_o);
-    return rc;
+    RG_GUARD(forward_impl(m, x, n, y));
 }
 
 // mean-squared-error gradient of one batch (no update): grads[MLP_NPARAM], loss
 int rg_mlp_gradient(rg_mlp* m, const float* x, const float* y, int n, float* grads, float* loss)
 {
     if (!m || n <= 0 || !x || !y || !grads) return set_error(RG_ERR_ARG, "bad argument");
-    std::vector<float> z = standardise(m, x, n);
-    float *d_x = nullptr, *d_y = nullptr;
-    int rc = dalloc(&d_x, z.size());
-    if (!rc) rc = dalloc(&d_y, (size_t)n);
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(d_x, z.data(), z.size() * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(d_y, y, n * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaMemsetAsync(m->d_g, 0, MLP_NPARAM * sizeof(float), m->st));
-    if (!rc) RG_CUDA_CHECK(cudaMemsetAsync(m->d_loss, 0, sizeof(float), m->st));
-    if (!rc) rc = run_tiles(m, true, d_x, d_y, nullptr, n, nullptr, 1.0f / (float)n);
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(grads, m->d_g, MLP_NPARAM * sizeof(float), cudaMemcpyDeviceToHost, m->st));
-    float l = 0.0f;
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(&l, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
-    if (loss) *loss = l;
-    cudaFree(d_x);
-    cudaFree(d_y);
-    return rc;
+    RG_GUARD(gradient_impl(m, x, y, n, grads, loss));
 }
 
 // AdamW training: `epochs` passes over the n samples in shuffled minibatches.
@@ -390,43 +635,7 @@ int rg_mlp_train(rg_mlp* m, const float* x, const float* y, int n, int epochs, i
 {
     if (!m || !x || !y || n <= 0 || epochs <= 0 || batch <= 0 || !(lr > 0.0f))
         return set_error(RG_ERR_ARG, "bad argument");
-    std::vector<float> z = standardise(m, x, n);
-    float *d_x = nullptr, *d_y = nullptr;
-    int* d_idx = nullptr;
-    int rc = dalloc(&d_x, z.size());
-    if (!rc) rc = dalloc(&d_y, (size_t)n);
-    if (!rc) rc = dalloc(&d_idx, (size_t)n);
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(d_x, z.data(), z.size() * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(d_y, y, n * sizeof(float), cudaMemcpyHostToDevice, m->st));
-    std::vector<int> idx(n);
-    for (int i = 0; i < n; i++) idx[i] = i;
-    std::mt19937_64 rng(seed);
-    float l = 0.0f;
-    const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    for (int ep = 0; ep < epochs && !rc; ep++) {
-        std::shuffle(idx.begin(), idx.end(), rng);
-        RG_CUDA_CHECK(cudaMemcpyAsync(d_idx, idx.data(), n * sizeof(int), cudaMemcpyHostToDevice, m->st));
-        for (int b0 = 0; b0 < n && !rc; b0 += batch) {
-            const int nb = std::min(batch, n - b0);
-            RG_CUDA_CHECK(cudaMemsetAsync(m->d_g, 0, MLP_NPARAM * sizeof(float), m->st));
-            RG_CUDA_CHECK(cudaMemsetAsync(m->d_loss, 0, sizeof(float), m->st));
-            rc = run_tiles(m, true, d_x, d_y, d_idx + b0, nb, nullptr, 1.0f / (float)nb);
-            if (rc) break;
-            m->step++;
-            const float bc1 = 1.0f - std::pow(b1, (float)m->step), bc2 = 1.0f - std::pow(b2, (float)m->step);
-            mlp_adamw_kernel<<<(MLP_NPARAM + 255) / 256, 256, 0, m->st>>>(m->d_w, m->d_m, m->d_v, m->d_g, MLP_NPARAM, lr,
-                                                                        b1, b2, eps, weight_decay, bc1, bc2);
-            RG_CUDA_CHECK(cudaGetLastError());
-            rc = sync_bf16(m);
-        }
-    }
-    if (!rc) RG_CUDA_CHECK(cudaMemcpyAsync(&l, m->d_loss, sizeof(float), cudaMemcpyDeviceToHost, m->st));
-    if (!rc) RG_CUDA_CHECK(cudaStreamSynchronize(m->st));
-    if (final_loss) *final_loss = l;
-    cudaFree(d_x);
-    cudaFree(d_y);
-    cudaFree(d_idx);
-    return rc;
+    RG_GUARD(train_impl(m, x, y, n, epochs, batch, lr, weight_decay, seed, final_loss));
 }
 
 }  // extern "C"

@@ -5,7 +5,7 @@ namespace redgb {
 
 constexpr int MLP_IN = 8;
 constexpr int MLP_HIDDEN = 64;
-constexpr int MLP_TB = 32;  // samples per CTA in the training kernels
+constexpr int MLP_TB = 64;  // samples per tile of the forward and training kernel
 constexpr int MLP_OFF_W1 = 0;
 constexpr int MLP_OFF_B1 = MLP_OFF_W1 + MLP_HIDDEN * MLP_IN;
 constexpr int MLP_OFF_W2 = MLP_OFF_B1 + MLP_HIDDEN;
