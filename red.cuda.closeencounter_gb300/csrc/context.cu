@@ -663,7 +663,9 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
         RG_CUDA_CHECK(cudaEventRecord(c->ev_fork, c->st));
         RG_CUDA_CHECK(cudaStreamWaitEvent(c->st2, c->ev_fork, 0));
     }
-    for (const auto& gr : c->plan[c->gravity_mode == RG_GRAVITY_MIXED ? 1 : 0]) {
+    const auto& groups = c->plan[c->gravity_mode == RG_GRAVITY_MIXED ? 1 : 0];
+    for (size_t ip = 0; ip < groups.size(); ip++) {
+        const auto& gr = groups[ip];
         g.tiles = c->d_tiles + gr.off;
         g.n_tiles = gr.n;
         switch (gr.kind) {
@@ -734,16 +736,29 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
                 c->n_kernels++;
             }
             if (!rc) {
-                const int src = c->tiles[gr.off].src_end - c->tiles[gr.off].src_begin;
-                const int src_tiles = (src + MIXED_SOURCE_TILE - 1) / MIXED_SOURCE_TILE;
-                int chunk;
-                if (c->mixed_chunk_src > 0) {
-                    chunk = std::min(c->mixed_chunk_src, src_tiles * MIXED_SOURCE_TILE);
-                } else {
-                    const int n = mixed_chunk_count(gr.n, src_tiles, c->n_sm);
-                    chunk = (src_tiles + n - 1) / n * MIXED_SOURCE_TILE;
+                // the mixed groups whose tiles follow on these (the interaction blocks): one launch
+                MixedGroups mg = MIXED_ONE_CHUNK;
+                int chunks = 1, n_tiles = gr.n, n_groups = 1;
+                while (n_groups < 3 && ip + n_groups < groups.size() && groups[ip + n_groups].kind == GROUP_MIXED &&
+                       groups[ip + n_groups].off == gr.off + (size_t)n_tiles)
+                    n_tiles += groups[ip + n_groups++].n;
+                for (int q = 0, end = 0; q < n_groups; q++) {
+                    const auto& gq = groups[ip + q];
+                    const int src = c->tiles[gq.off].src_end - c->tiles[gq.off].src_begin;
+                    const int src_tiles = (src + MIXED_SOURCE_TILE - 1) / MIXED_SOURCE_TILE;
+                    int chunk;
+                    if (c->mixed_chunk_src > 0) {
+                        chunk = std::min(c->mixed_chunk_src, src_tiles * MIXED_SOURCE_TILE);
+                    } else {
+                        const int n = mixed_chunk_count(n_tiles, src_tiles, c->n_sm);
+                        chunk = (src_tiles + n - 1) / n * MIXED_SOURCE_TILE;
+                    }
+                    mg.end[q] = end += gq.n;
+                    mg.chunk[q] = chunk;
+                    chunks = std::max(chunks, (src + chunk - 1) / chunk);
                 }
-                const int chunks = (src + chunk - 1) / chunk;
+                g.n_tiles = n_tiles;
+                ip += n_groups - 1;
                 if (chunks > 1 && (size_t)chunks * 3 * c->cap > c->partial_cap && c->capturing) {
                     c->capture_failed = true;  // allocate outside a capture (the next direct run)
                     rc = RG_ERR_STATE;
@@ -755,7 +770,7 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
                     if (!rc) c->partial_cap = (size_t)chunks * 3 * c->cap;
                 }
                 if (!rc)
-                    rc = launch_grav_mixed_tiles(g, c->d_split, c->d_heavy + gr.off, c->near_ratio, chunks, chunk,
+                    rc = launch_grav_mixed_tiles(g, c->d_split, c->d_heavy + gr.off, c->near_ratio, chunks, mg,
                                                  c->d_partial, c->cap, c->d_kerr, c->hold_tile_copies != 0, c->st);
                 c->n_kernels += chunks > 1;
             }

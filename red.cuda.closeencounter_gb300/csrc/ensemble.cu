@@ -1389,7 +1389,7 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
             if (!rc) {
                 // one source chunk: the disks' source counts differ, so a chunked split would
                 // need a partial buffer per disk
-                rc = launch_grav_mixed_tiles(g, e->d_split, e->d_heavy + gr.off, e->near_ratio, 1, MIXED_SOURCE_TILE,
+                rc = launch_grav_mixed_tiles(g, e->d_split, e->d_heavy + gr.off, e->near_ratio, 1, MIXED_ONE_CHUNK,
                                              nullptr, e->cap, e->d_kerr, false, e->st);
                 e->n_kernels++;
             }

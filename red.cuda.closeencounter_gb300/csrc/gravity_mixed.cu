@@ -150,8 +150,8 @@ struct MixedArgs {
     const SplitPos* sp;
     const int* heavy_end;  // per tile: sources [src_begin, heavy_end) are heavy
     float near_ratio;
-    int chunk;             // sources per grid.y chunk (multiple of MX_T)
-    double* partial;       // n_chunks x 3 x n_part doubles, or nullptr when grid.y == 1
+    MixedGroups groups;    // sources per grid.y chunk (multiples of MX_T)
+    double* partial;       // grid.y x 3 x n_part doubles, or nullptr when grid.y == 1
     int n_part;            // row length of `partial`
     unsigned int* err;     // set to 1 when a tile copy did not arrive within the wait limit
     int hold;              // test hook: issue no tile copies (the waits run out)
@@ -528,8 +528,10 @@ __global__ void __launch_bounds__(256, 2) grav_mixed_kernel(MixedArgs a)
     if (g.sys_active && !g.sys_active[tile.sys]) return;
     const int heavy_end = a.heavy_end[blockIdx.x];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int src_lo = tile.src_begin + blockIdx.y * a.chunk;
-    const int src_hi = min(tile.src_end, src_lo + a.chunk);
+    const int chunk = a.groups.chunk_of(blockIdx.x);
+    const int src_lo = tile.src_begin + blockIdx.y * chunk;
+    if (blockIdx.y > 0 && src_lo >= tile.src_end) return;  // another group has more chunks
+    const int src_hi = min(tile.src_end, src_lo + chunk);
     const int first = max(heavy_end, src_lo);
     const int n_tiles = first < src_hi ? (src_hi - first + MX_T - 1) / MX_T : 0;
 
@@ -778,23 +780,24 @@ __global__ void __launch_bounds__(256, 2) grav_mixed_kernel(MixedArgs a)
 }
 
 // a_i = sum over source chunks of the partials, in chunk order
-__global__ void mixed_reduce_kernel(const double* __restrict__ partial, int n_chunks, int n_part, const Tile* tiles,
-                                    int n_tiles, const int* sys_active, double* ax, double* ay, double* az,
+__global__ void mixed_reduce_kernel(const double* __restrict__ partial, MixedGroups groups, int n_part,
+                                    const Tile* tiles, const int* sys_active, double* ax, double* ay, double* az,
                                     int acc_f2)
 {
     const Tile tile = tiles[blockIdx.x];
     if (sys_active && !sys_active[tile.sys]) return;
-    const int i = tile.sink_begin + threadIdx.x;
+    const int i = tile.sink_begin + threadIdx.x, comp = blockIdx.y;
     if (i >= tile.sink_end) return;
-    for (int comp = 0; comp < 3; comp++) {
-        double v = 0.0;
-        for (int c = 0; c < n_chunks; c++) v += partial[((long long)c * 3 + comp) * n_part + i];
-        double* row = comp == 0 ? ax : (comp == 1 ? ay : az);
-        if (acc_f2)
-            reinterpret_cast<float2*>(row)[i] = to_f2(v);
-        else
-            row[i] = v;
-    }
+    const int chunk = groups.chunk_of(blockIdx.x);
+    const int n_chunks = max(1, (tile.src_end - tile.src_begin + chunk - 1) / chunk);
+    double v = 0.0;
+#pragma unroll 8
+    for (int c = 0; c < n_chunks; c++) v += partial[((long long)c * 3 + comp) * n_part + i];
+    double* row = comp == 0 ? ax : (comp == 1 ? ay : az);
+    if (acc_f2)
+        reinterpret_cast<float2*>(row)[i] = to_f2(v);
+    else
+        row[i] = v;
 }
 
 // Row kernel: one thread per sink, the tile's sources (a few massive bodies) staged in
@@ -1396,8 +1399,8 @@ int launch_split_positions(const double* x, const double* y, const double* z, co
 }
 
 int launch_grav_mixed_tiles(const GravArgs& g, const void* split, const int* heavy_end, float near_ratio,
-                            int n_chunks, int chunk, double* partial, int n_part, unsigned int* err, bool hold,
-                            cudaStream_t st)
+                            int n_chunks, const MixedGroups& groups, double* partial, int n_part, unsigned int* err,
+                            bool hold, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
     constexpr int smem = (int)sizeof(MixedSmem);
@@ -1417,7 +1420,7 @@ int launch_grav_mixed_tiles(const GravArgs& g, const void* split, const int* hea
     a.sp = (const SplitPos*)split;
     a.heavy_end = heavy_end;
     a.near_ratio = near_ratio;
-    a.chunk = n_chunks > 1 ? chunk : (1 << 30);
+    a.groups = groups;
     a.partial = n_chunks > 1 ? partial : nullptr;
     a.n_part = n_part;
     a.hold = hold ? 1 : 0;
@@ -1428,8 +1431,8 @@ int launch_grav_mixed_tiles(const GravArgs& g, const void* split, const int* hea
         grav_mixed_kernel<false><<<grid, 256, smem, st>>>(a);
     RG_CUDA_CHECK(cudaGetLastError());
     if (n_chunks > 1) {
-        mixed_reduce_kernel<<<g.n_tiles, MX_S, 0, st>>>(partial, n_chunks, n_part, g.tiles, g.n_tiles, g.sys_active,
-                                                        g.ax, g.ay, g.az, g.acc_f2);
+        mixed_reduce_kernel<<<dim3(g.n_tiles, 3), MX_S, 0, st>>>(partial, groups, n_part, g.tiles, g.sys_active, g.ax,
+                                                                 g.ay, g.az, g.acc_f2);
         RG_CUDA_CHECK(cudaGetLastError());
     }
     return 0;

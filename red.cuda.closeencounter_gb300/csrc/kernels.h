@@ -115,9 +115,17 @@ int launch_split_positions(const double* x, const double* y, const double* z, co
                            float2* mass_f2 = nullptr);
 constexpr int SCREEN_MAX_WORDS = 4;  // GravArgs::smax per system: radius, mass, star distance, spare
 // hold: test hook -- no tile copies are issued, so the kernel's bounded waits run out
+// tiles of up to three groups (interaction blocks) in one launch: tile t is of the first group
+// whose `end` is above t (after the last group: 1 << 30); chunk: sources per grid.y chunk
+struct MixedGroups {
+    int end[3], chunk[3];
+    __host__ __device__ int chunk_of(int t) const { return t < end[0] ? chunk[0] : (t < end[1] ? chunk[1] : chunk[2]); }
+};
+constexpr MixedGroups MIXED_ONE_CHUNK{{1 << 30, 1 << 30, 1 << 30}, {1 << 30, 1 << 30, 1 << 30}};
+// n_chunks: the most chunks of a group (grid.y)
 int launch_grav_mixed_tiles(const GravArgs& g, const void* split, const int* heavy_end, float near_ratio,
-                            int n_chunks, int chunk, double* partial, int n_part, unsigned int* err, bool hold,
-                            cudaStream_t st);
+                            int n_chunks, const MixedGroups& groups, double* partial, int n_part, unsigned int* err,
+                            bool hold, cudaStream_t st);
 // heavy pairs of the mixed-precision mode in double-float arithmetic (gravity_mixed.cu):
 // the row kernel for blocks with a few massive sources, the few-sink kernel for the
 // star's and giants' own rows (partial: 3 x rows x pitch doubles, pitch >= source chunks)

@@ -36,3 +36,27 @@ def test_mixed_tile_edges(gpulib, n):
         am = g.calc_accel()
         err = np.linalg.norm(np.stack([am[f] for f in "xyz"], 1) - a_e, axis=1)
         assert (err <= tol).all(), (n, chunk, float((err / tol).max()))
+
+
+@pytest.mark.parametrize("n_emb,n_pl,n_tp", [(70, 1, 1), (100, 129, 0), (130, 0, 300), (300, 700, 257)])
+def test_blocks_in_one_launch(gpulib, n_emb, n_pl, n_tp):
+    """The three interaction blocks' tiles in one launch, each block with its own source count
+    and chunks."""
+    rng = np.random.RandomState(n_emb)
+    emb = [(10.0 ** rng.uniform(-9, -7), 1.0 + 3.0 * k / n_emb, 0.02) for k in range(n_emb)]
+    disk = bodies.make_disk(n_pl=n_pl, embryos=emb, giants=((9.55e-4, 5.2, 0.05),), n_tp=n_tp, seed=n_pl)
+    g = lib.System(disk, bodies.thresholds())
+    ref = g.calc_accel()
+    a_e = np.stack([ref[f] for f in "xyz"], 1)
+    m = disk.p["mass"].copy()
+    m[:2] = 0.0
+    r = np.stack([disk.r[f] for f in "xyz"], 1)
+    d2 = ((r[:, None] - r[None]) ** 2).sum(-1)
+    np.fill_diagonal(d2, np.inf)
+    tol = 2.0 ** -20 * (m[None] / d2).sum(1) + 2.0 ** -42 * np.linalg.norm(a_e, axis=1)
+    g.set_gravity_mode(T.GRAVITY_MIXED)
+    for chunk in (0, 256, 512):
+        g.set_launch_shape(mixed_chunks=chunk)
+        am = g.calc_accel()
+        err = np.linalg.norm(np.stack([am[f] for f in "xyz"], 1) - a_e, axis=1)
+        assert (err <= tol).all(), (chunk, float((err / tol).max()))
