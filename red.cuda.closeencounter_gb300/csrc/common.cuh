@@ -94,6 +94,7 @@ struct GravArgs {
     // velocity rows (stages after the step start)
     int acc_f2;
     int vel_f2;
+    int i_shift;  // added to a record's sink index (kernels with a CTA's own body numbering), else 0
 };
 
 // the collision factor of a tile's system

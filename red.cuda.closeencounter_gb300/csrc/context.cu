@@ -147,6 +147,7 @@ struct rg_ctx {
         int max_sinks;  // few-sink groups: widest tile
     };
     std::vector<Group> plan[2];
+    bool swarm = false;  // a disk for swarm_step.cu
     std::vector<Tile> tiles;       // all groups' tiles, uploaded to d_tiles
     std::vector<int> heavy_mx;     // per tile (mixed groups): end of the heavy sources
     std::vector<int> screen_slot;  // per body: 0 light, -1 heavy (the mixed kernels' screen cutoffs)
@@ -410,7 +411,10 @@ void build_tiles(rg_ctx* c)
     // balanced tiles, each one part of the heavy rows
     const bool sym = !src0 && nsi >= 1 && nsi <= DF_SYM_MAX_HEAVY && nm > nsi && nsi <= c->rowseq_max_src &&
                      nm > c->rowseq_max_src && nsi <= FEW_BLOCK_SINKS;
-    const int sym_ctas = sym ? std::min((nm - nsi + DF_SYM_PASS - 1) / DF_SYM_PASS, DF_SYM_RESIDENT * c->n_sm) : 0;
+    // (a disk whose RKF7(8) steps swarm_step.cu takes has that kernel's slices as segments)
+    c->swarm = sym && nt == nm && swarm_step_fits(nsi, nm - nsi);
+    const int sym_unit = c->swarm ? swarm_slice(nm - nsi) : DF_SYM_PASS;
+    const int sym_ctas = sym ? std::min((nm - nsi + sym_unit - 1) / sym_unit, DF_SYM_RESIDENT * c->n_sm) : 0;
     c->sym_cta.clear();
     auto add_group = [&](int mode, int kind, int s0, int s1, int src1, int block, int step) {
         if (s1 <= s0) return;
@@ -457,8 +461,8 @@ void build_tiles(rg_ctx* c)
             if (sym && b.block == 1) {  // the heavy rows [0, nsi), then one segment per CTA (Tile::part from 1)
                 const size_t t0 = c->tiles.size();
                 std::vector<int> parts;
-                build_sym_segments({Tile{b.s0, b.s1, 0, nsi, 0, 0, b.block, 0}}, sym_ctas, DF_SYM_PASS,
-                                   DF_SYM_SEGMENT_COST, c->tiles, c->sym_cta, parts);
+                build_sym_segments({Tile{b.s0, b.s1, 0, nsi, 0, 0, b.block, 0}}, sym_ctas, sym_unit,
+                                   c->swarm ? 0.0 : DF_SYM_SEGMENT_COST, c->tiles, c->sym_cta, parts);
                 const int nseg = (int)(c->tiles.size() - t0);
                 rg_ctx::Group gr{GROUP_DF_SYM, t0, nseg, c->few_rows, nsi, nsi, 0};
                 const int row0 = c->few_rows;
@@ -1284,8 +1288,9 @@ bool replay_step_graph(rg_ctx* c, rg_ctx::StepGraph& sg, F body, int* rc)
     return true;
 }
 
-// A step of a small system: each attempt one kernel (small_step.cu), one synchronisation
-int step_rkf78_small(rg_ctx* c)
+// A step of a small system or a planetesimal disk: each attempt one kernel (small_step.cu,
+// swarm_step.cu), one synchronisation
+int step_rkf78_small(rg_ctx* c, bool swarm)
 {
     SmallStepArgs a{};
     a.g.mass = c->d_mass;
@@ -1293,6 +1298,8 @@ int step_rkf78_small(rg_ctx* c)
     a.g.id = c->d_id;
     a.g.f_rad = c->thr[RG_THRESHOLD_RADII_ENHANCE_FACTOR];
     a.g.hill_f3 = c->hill_factor * c->hill_factor * c->hill_factor;
+    a.g.f_rad_f = (float)a.g.f_rad;
+    a.g.hill_f3_f = (float)a.g.hill_f3;
     a.g.record = (c->inner_steps && a.g.f_rad > 0.0) ? 1 : 0;
     a.g.hill = c->hill_factor > 0.0 ? 1 : 0;
     a.g.ev = EventBuf{c->d_ev, c->d_ev_count, c->ev_cap};
@@ -1329,7 +1336,7 @@ int step_rkf78_small(rg_ctx* c)
         a.dt = c->dt_try;
         a.first = iter == 0;
         a.attempt = (unsigned int)iter;
-        const int rc = launch_small_rkf78(a, c->st);
+        const int rc = swarm ? launch_swarm_rkf78(a, c->st) : launch_small_rkf78(a, c->st);
         if (rc) return rc;
         c->n_kernels++;
         const int evals = c->r_max - 1 + (iter == 0);
@@ -1354,11 +1361,15 @@ int step_rkf78_small(rg_ctx* c)
 
 int step_rkf78(rg_ctx* c)
 {
-    // (up to SMALL_MAX bodies one SM is faster than a kernel per stage; timing hooks take the latter)
-    if (c->gravity_mode == RG_GRAVITY_FP64 && c->frame == RG_FRAME_BARY && c->n_total() <= SMALL_MAX && c->n_total() > 0 &&
-        !c->profiling && c->use_graphs) {
+    // (up to SMALL_MAX bodies one SM, and up to SWARM_MAX_LIGHT planetesimals one cluster are faster
+    // than a kernel per stage: 45 against 281 us an attempt of nine bodies in FP64, 88 against 247 us
+    // of 1027 in mixed precision; timing and test hooks take the latter)
+    const bool small = c->gravity_mode == RG_GRAVITY_FP64 && c->frame == RG_FRAME_BARY && c->n_total() <= SMALL_MAX &&
+                       c->n_total() > 0;
+    const bool swarm = c->gravity_mode == RG_GRAVITY_MIXED && c->swarm;
+    if ((small || swarm) && !c->profiling && c->use_graphs && !c->hold_tile_copies) {
         c->attempt_dt.clear();
-        return step_rkf78_small(c);
+        return step_rkf78_small(c, swarm);
     }
     const size_t cap = (size_t)c->cap;
     c->attempt_dt.clear();

@@ -177,6 +177,12 @@ struct SmallStepArgs {
     StepResult* out;
 };
 int launch_small_rkf78(const SmallStepArgs& a, cudaStream_t st);
+// ... and of a planetesimal disk in mixed precision: a few heavy bodies (SI, at most
+// DF_SYM_MAX_HEAVY) and at most SWARM_MAX_LIGHT light ones (NSI), nothing else (swarm_step.cu)
+constexpr int SWARM_MAX_LIGHT = 3072;
+int swarm_slice(int n_light);
+bool swarm_step_fits(int n_heavy, int n_light);
+int launch_swarm_rkf78(const SmallStepArgs& a, cudaStream_t st);
 
 int measure_pipe_peak(int kind, double* tflops);
 

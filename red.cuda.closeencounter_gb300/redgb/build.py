@@ -32,6 +32,7 @@ UNITS = {
     "gravity_cert.cu": ["-fmad=false"],
     "small_step.cu": ["-fmad=false"],
     "gravity_mixed.cu": [],
+    "swarm_step.cu": [],
     "ensemble.cu": ["-fmad=false"],
     "mlp.cu": [],
     "noalloc.cu": ["-fmad=false"],
