@@ -147,7 +147,7 @@ struct rg_ctx {
         int max_sinks;  // few-sink groups: widest tile
     };
     std::vector<Group> plan[2];
-    bool swarm = false;  // a disk for swarm_step.cu
+    bool swarm = false, swarm_fp64 = false;  // a disk for swarm_step.cu, swarm_fp64.cu
     std::vector<Tile> tiles;       // all groups' tiles, uploaded to d_tiles
     std::vector<int> heavy_mx;     // per tile (mixed groups): end of the heavy sources
     std::vector<int> screen_slot;  // per body: 0 light, -1 heavy (the mixed kernels' screen cutoffs)
@@ -413,6 +413,7 @@ void build_tiles(rg_ctx* c)
                      nm > c->rowseq_max_src && nsi <= FEW_BLOCK_SINKS;
     // (a disk whose RKF7(8) steps swarm_step.cu takes has that kernel's slices as segments)
     c->swarm = sym && nt == nm && swarm_step_fits(nsi, nm - nsi);
+    c->swarm_fp64 = sym && nt == nm && swarm_fp64_fits(nsi, nm - nsi);
     const int sym_unit = c->swarm ? swarm_slice(nm - nsi) : DF_SYM_PASS;
     const int sym_ctas = sym ? std::min((nm - nsi + sym_unit - 1) / sym_unit, DF_SYM_RESIDENT * c->n_sm) : 0;
     c->sym_cta.clear();
@@ -1289,7 +1290,7 @@ bool replay_step_graph(rg_ctx* c, rg_ctx::StepGraph& sg, F body, int* rc)
 }
 
 // A step of a small system or a planetesimal disk: each attempt one kernel (small_step.cu,
-// swarm_step.cu), one synchronisation
+// swarm_step.cu, swarm_fp64.cu), one synchronisation
 int step_rkf78_small(rg_ctx* c, bool swarm)
 {
     SmallStepArgs a{};
@@ -1336,7 +1337,9 @@ int step_rkf78_small(rg_ctx* c, bool swarm)
         a.dt = c->dt_try;
         a.first = iter == 0;
         a.attempt = (unsigned int)iter;
-        const int rc = swarm ? launch_swarm_rkf78(a, c->st) : launch_small_rkf78(a, c->st);
+        const int rc = !swarm ? launch_small_rkf78(a, c->st)
+                              : (c->gravity_mode == RG_GRAVITY_MIXED ? launch_swarm_rkf78(a, c->st)
+                                                                     : launch_swarm_rkf78_fp64(a, c->st));
         if (rc) return rc;
         c->n_kernels++;
         const int evals = c->r_max - 1 + (iter == 0);
@@ -1362,11 +1365,11 @@ int step_rkf78_small(rg_ctx* c, bool swarm)
 int step_rkf78(rg_ctx* c)
 {
     // (up to SMALL_MAX bodies one SM, and up to SWARM_MAX_LIGHT planetesimals one cluster are faster
-    // than a kernel per stage: 45 against 281 us an attempt of nine bodies in FP64, 88 against 247 us
-    // of 1027 in mixed precision; timing and test hooks take the latter)
+    // than a kernel per stage: 45 against 281 us an attempt of nine bodies in FP64, 189 against 420 us
+    // of 1027 in FP64 and 88 against 247 us in mixed precision; timing and test hooks take the latter)
     const bool small = c->gravity_mode == RG_GRAVITY_FP64 && c->frame == RG_FRAME_BARY && c->n_total() <= SMALL_MAX &&
                        c->n_total() > 0;
-    const bool swarm = c->gravity_mode == RG_GRAVITY_MIXED && c->swarm;
+    const bool swarm = c->gravity_mode == RG_GRAVITY_MIXED ? c->swarm : (!small && c->swarm_fp64);
     if ((small || swarm) && !c->profiling && c->use_graphs && !c->hold_tile_copies) {
         c->attempt_dt.clear();
         return step_rkf78_small(c, swarm);

@@ -183,6 +183,8 @@ constexpr int SWARM_MAX_LIGHT = 3072;
 int swarm_slice(int n_light);
 bool swarm_step_fits(int n_heavy, int n_light);
 int launch_swarm_rkf78(const SmallStepArgs& a, cudaStream_t st);
+bool swarm_fp64_fits(int n_heavy, int n_light);  // the same disks in FP64 (swarm_fp64.cu)
+int launch_swarm_rkf78_fp64(const SmallStepArgs& a, cudaStream_t st);
 
 int measure_pipe_peak(int kind, double* tflops);
 

@@ -11,26 +11,11 @@ struct PairOut {
     double tx, ty, tz;
 };
 
-// One (sink, source) pair: the term added to a_i and the event tests of pp_disk.cu:265
-// (radius criterion) and of the mutual Hill sphere (cube form, no cube root).
-// EVENTS = false: the term alone, for a pair whose event tests another evaluation has made.
-// PIPE: the square root and the division on the FP64 pipe (the same bits), where the pipe has
-// room and the integer pipes have not.
-template <bool EVENTS = true, bool PIPE = false>
-__device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, int i, int j, double xi, double yi,
-                                          double zi, double Ri, double mi, double rhoi, double xj, double yj,
-                                          double zj, double mj, double Rj, double rhoj, PairOut& o)
+// the event tests of a pair at distance d and their records
+__device__ __forceinline__ void pair_events(const GravArgs& g, const Tile& tile, int i, int j, double xi, double yi,
+                                            double zi, double Ri, double mi, double rhoi, double xj, double yj,
+                                            double zj, double mj, double Rj, double rhoj, double d)
 {
-    const double dx = xj - xi;
-    const double dy = yj - yi;
-    const double dz = zj - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    const double d = PIPE ? __dsqrt_rn(r2) : rn_sqrt(r2);  // rn_*: on the integer pipes (exact_fp64.h)
-    const double w = PIPE ? __ddiv_rn(mj, d * r2) : rn_div(mj, d * r2);
-    o.tx = w * dx;
-    o.ty = w * dy;
-    o.tz = w * dz;
-    if (!EVENTS) return;
     const int li = i - tile.base, lj = j - tile.base;
     bool rad = g.record && li > 0 && li > lj && d < tile_f_rad(g, tile) * (Ri + Rj);
     bool hill = false;
@@ -50,7 +35,7 @@ __device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, i
                 DevEvent* e = &eb.rec[slot];
                 e->seq = record_seq(g, tile, kind);
                 e->kind = kind;
-                e->i = i;
+                e->i = i + g.i_shift;
                 e->j = j;
                 e->sys = tile.sys;
                 e->pad = 0;
@@ -66,6 +51,28 @@ __device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, i
             }
         }
     }
+}
+
+// One (sink, source) pair: the term added to a_i and the event tests of pp_disk.cu:265
+// (radius criterion) and of the mutual Hill sphere (cube form, no cube root).
+// EVENTS = false: the term alone, for a pair whose event tests another evaluation has made.
+// PIPE: the square root and the division on the FP64 pipe (the same bits), where the pipe has
+// room and the integer pipes have not.
+template <bool EVENTS = true, bool PIPE = false>
+__device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, int i, int j, double xi, double yi,
+                                          double zi, double Ri, double mi, double rhoi, double xj, double yj,
+                                          double zj, double mj, double Rj, double rhoj, PairOut& o)
+{
+    const double dx = xj - xi;
+    const double dy = yj - yi;
+    const double dz = zj - zi;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double d = PIPE ? __dsqrt_rn(r2) : rn_sqrt(r2);  // rn_*: on the integer pipes (exact_fp64.h)
+    const double w = PIPE ? __ddiv_rn(mj, d * r2) : rn_div(mj, d * r2);
+    o.tx = w * dx;
+    o.ty = w * dy;
+    o.tz = w * dz;
+    if (EVENTS) pair_events(g, tile, i, j, xi, yi, zi, Ri, mi, rhoi, xj, yj, zj, mj, Rj, rhoj, d);
 }
 
 }  // namespace redgb

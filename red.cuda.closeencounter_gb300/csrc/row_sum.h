@@ -102,6 +102,30 @@ XF_HD uint32_t row_code(uint32_t rec, uint64_t ut)
     return (uint32_t)p | (uint32_t)k << 5 | even << 8 | n << 9 | g << 17;
 }
 
+// A code unpacked for a run through many of them, with `in` added to the offset before it: d becomes
+// (v + half + (v >> k & even)) >> k with v = d 2^p + n.  Offsets of any size, as long as v keeps to
+// 2^29 (`most` collects its bits, all of them where d 2^p does not fit 32 bits).
+struct RowRule {
+    int n, half, shifts, even;  // shifts: p | k << 16
+};
+XF_HD bool row_rule(uint32_t code, int in, RowRule* r)
+{
+    const int p = (int)(code & 31u), k = (int)(code >> 5 & 7u), even = (int)(code >> 8 & 1u);
+    const int64_t n = (int64_t)(code >> 9 & 0xffu) + (int64_t)in * (1 << p);
+    r->n = (int)n;
+    r->half = ((1 << k) >> 1) - even - (int)(code >> 17) * (1 << k);
+    r->shifts = p | k << 16;
+    r->even = even;
+    return n < (1 << 29) && n > -(1 << 29);
+}
+XF_HD int row_follow(const RowRule& r, int d, int* most)
+{
+    const int k = r.shifts >> 16, p = r.shifts & 31;
+    const int v0 = (int)((uint32_t)d << p), v = v0 + r.n;
+    *most |= (v0 ^ (v0 >> 31)) | ((v0 >> p) == d ? 0 : INT_MAX);
+    return (v + r.half + (v >> k & r.even)) >> k;
+}
+
 // the offset after an addition with this code, |d| < MAX_OFF
 XF_HD int row_apply(uint32_t code, int d)
 {
@@ -136,14 +160,14 @@ XF_HD uint64_t row_from_units(int64_t u, int top)
 // the double d ulps above x in value (|d| small, x not near its binade's ends)
 XF_HD uint64_t row_shift(uint64_t u, int d) { return (u >> 63) ? u - (uint64_t)(int64_t)d : u + (uint64_t)(int64_t)d; }
 
-// x - y in ulps for x, y of one sign and binade with a difference below MAX_OFF; false otherwise
-XF_HD bool row_diff(uint64_t x, uint64_t y, int* d)
+// x - y in ulps for x, y of one sign and binade with a difference below `limit`; false otherwise
+XF_HD bool row_diff(uint64_t x, uint64_t y, int* d, int64_t limit = MAX_OFF)
 {
     *d = 0;
     if (x == y) return true;
     if ((x >> 52) != (y >> 52) || ((x >> 52) & 0x7ff) == 0 || ((x >> 52) & 0x7ff) == 2047) return false;
     const int64_t v = (x >> 63) ? (int64_t)(y - x) : (int64_t)(x - y);
-    if (v >= MAX_OFF || v <= -MAX_OFF) return false;
+    if (v >= limit || v <= -limit) return false;
     *d = (int)v;
     return true;
 }
@@ -153,6 +177,7 @@ XF_HD bool row_diff(uint64_t x, uint64_t y, int* d)
 #if defined(__CUDACC__)
 
 constexpr int ROW_SEG_MAX = 36;  // terms per lane and call
+constexpr int ROW_CTA_WARPS = 16;  // most warps of cta_row_sum
 
 // acc + T_0 + ... + T_{m-1}, rounded after every addition in that order, m <= 32 seg,
 // seg <= ROW_SEG_MAX: term e is at T[e / seg * pitch + e % seg].  Every lane of the warp calls
@@ -312,6 +337,164 @@ __device__ __forceinline__ double warp_row_sum(double acc, const double* T, int 
     }
     const uint64_t mine = done ? tend : rs::row_shift(end, P + off);
     return __longlong_as_double((long long)__shfl_sync(ALL, (unsigned long long)mine, 31));
+}
+
+// The same sum by all W warps of a CTA (blockDim.x = 32 W), each lane one of 32 W segments: the
+// lanes' passes get as many times shorter, the codes are still applied in order, by the first
+// warp, one after the other from one list.  Terms T[0 .. m) in shared memory, m <= 32 W
+// ROW_SEG_MAX; every thread of the CTA calls this and gets the sum.  A slow lane is added again
+// from its true start when its turn comes; a row with too many of them, or with offsets out of
+// range, is summed by the first warp alone.
+// Measured: a hovering row of 1027 terms (some 250 codes) 15.5 k cycles of eight warps,
+// warp_row_sum 28 k.
+constexpr int ROW_RULES = 1024;  // most codes of a row that are applied
+constexpr int ROW_HARD = 8;      // most lanes of a row that are added again
+struct CtaRowSmem {
+    rs::RowRule rule[ROW_RULES];
+    struct {
+        int lane, rule, in;  // the lane, its place among the rules, the offset's change since the lane with codes before
+        unsigned long long before, end;
+    } hard[ROW_HARD];
+    int P[32 * ROW_CTA_WARPS];  // of the lanes with codes
+    int top[ROW_CTA_WARPS];
+    long long units[ROW_CTA_WARPS];
+    unsigned long long end[ROW_CTA_WARPS], last;
+    int diff[ROW_CTA_WARPS], count[ROW_CTA_WARPS], coded[ROW_CTA_WARPS];
+    int last_in;
+    double sum;
+};
+
+// codes: max(m, 32 ROW_SEG_MAX) entries at least
+__device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* codes, CtaRowSmem& S)
+{
+    constexpr unsigned ALL = 0xffffffffu;
+    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, me = threadIdx.x;
+    const int seg = (m + 32 * W - 1) / (32 * W);
+    const int n = max(0, min(seg, m - me * seg));
+    const double* const t = T + me * seg;
+    int top = 0;
+    for (int k = 0; k < n; k++) top = max(top, (int)((uint32_t)(xf::dbits(t[k]) >> 52) & 0x7ffu));
+    top = __reduce_max_sync(ALL, top);
+    if (lane == 0) S.top[warp] = top;
+    __syncthreads();
+    for (int w = 0; w < W; w++) top = max(top, S.top[w]);
+    long long u = 0;
+    for (int k = 0; k < n; k++) u += rs::row_units(xf::dbits(t[k]), top);
+    const long long own = u;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const long long o = __shfl_up_sync(ALL, u, off);
+        if (lane >= off) u += o;
+    }
+    if (lane == 31) S.units[warp] = u;
+    __syncthreads();
+    long long base = u - own;
+    for (int w = 0; w < warp; w++) base += S.units[w];
+    double a = __longlong_as_double((long long)rs::row_from_units(base, top));  // (the first lane: 0.0)
+    const uint64_t guess = xf::dbits(a);
+    bool hard = rs::near_edge(guess);
+    int nc = 0;
+    uint32_t* const code = codes + me * seg;
+    for (int k = 0; k < n; k++) {
+        const double tk = t[k], s = __dadd_rn(a, tk);
+        const uint32_t rec = rs::row_mark(xf::dbits(a), xf::dbits(tk), xf::dbits(s), k, &hard);
+        if (rec) code[nc++] = rec;
+        a = s;
+    }
+    for (int q = 0; q < nc; q++) code[q] = rs::row_code(code[q], xf::dbits(t[code[q] >> 13 & 63u]));
+    const uint64_t end = xf::dbits(a);
+    if (lane == 31) S.end[warp] = end;
+    if (me == (int)blockDim.x - 1) S.last = end;
+    __syncthreads();
+    uint64_t before = __shfl_up_sync(ALL, (unsigned long long)end, 1);
+    if (lane == 0 && warp > 0) before = S.end[warp - 1];
+    int d = 0;
+    bool loose = !rs::row_diff(before, guess, &d, 1 << 20);
+    if (me == 0) {
+        loose = false;
+        d = 0;
+    }
+    if (!__syncthreads_or(loose || d != 0)) return __longlong_as_double((long long)S.last);
+    // the lanes' offsets if none had codes, and where a lane's codes stand among all (the first
+    // lane's change nothing: its offset is 0)
+    const bool again = me > 0 && (hard || loose), has = me > 0 && (again || nc > 0);
+    const int mine = again ? 1 : (me > 0 ? nc : 0);
+    int P = d, at = mine | (again ? 1 << 20 : 0), order = has;  // at: above bit 20 the slow lanes
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const int o = __shfl_up_sync(ALL, P, off), oc = __shfl_up_sync(ALL, at, off), oo = __shfl_up_sync(ALL, order, off);
+        if (lane >= off) {
+            P += o;
+            at += oc;
+            order += oo;
+        }
+    }
+    if (lane == 31) {
+        S.diff[warp] = P;
+        S.count[warp] = at;
+        S.coded[warp] = order;
+    }
+    __syncthreads();
+    int total = 0;
+    for (int w = 0; w < W; w++) {
+        if (w < warp) {
+            P += S.diff[w];
+            at += S.count[w];
+            order += S.coded[w];
+        }
+        total += S.count[w];
+    }
+    const int n_hard = total >> 20, n_rule = total & 0xfffff;
+    if (has) S.P[order - 1] = P;
+    bool slow = __syncthreads_or(n_rule > ROW_RULES || n_hard > ROW_HARD);
+    const int since = P - (order - (int)has > 0 ? S.P[order - (int)has - 1] : 0);
+    if (me == (int)blockDim.x - 1) S.last_in = has ? 0 : since;
+    bool fit = true;
+    if (!slow && has) {
+        const int first = (at & 0xfffff) - mine;
+        if (again) {
+            auto& h = S.hard[(at >> 20) - 1];
+            h.lane = me;
+            h.rule = first;
+            h.in = since - d;
+            h.before = before;
+            h.end = end;
+        } else {
+            for (int q = 0; q < nc; q++) fit = rs::row_rule(code[q], q == 0 ? since : 0, &S.rule[first + q]) && fit;
+        }
+    }
+    constexpr int LIM = 1 << 29;
+    slow = __syncthreads_or(slow || !fit);
+    if (warp == 0) {
+        int off = 0, most = slow ? LIM : 0;
+        uint64_t tend = 0;  // the true end of the last lane added again
+        int q = 0;
+        for (int k = 0; k <= n_hard && !slow; k++) {
+            const int to = k < n_hard ? S.hard[k].rule : n_rule;
+#pragma unroll 4
+            for (; q < to; q++) off = rs::row_follow(S.rule[q], off, &most);
+            if (k == n_hard || most >= LIM) break;
+            const auto& h = S.hard[k];
+            const bool follows = k > 0 && S.hard[k - 1].lane == h.lane - 1;
+            double b = __longlong_as_double((long long)(follows ? tend : rs::row_shift(h.before, off + h.in)));
+            for (int e = h.lane * seg; e < min(m, h.lane * seg + seg); e++) b = __dadd_rn(b, T[e]);
+            tend = xf::dbits(b);
+            if (!rs::row_diff(tend, h.end, &off, LIM)) most = LIM;
+            q = to + 1;
+        }
+        double sum = 0.0;
+        if (most < LIM) {
+            sum = __longlong_as_double((long long)rs::row_shift(S.last, off + S.last_in));
+        } else {  // (the codes' space is free: they are not used)
+            for (int k = 0; k < m; k += 32 * ROW_SEG_MAX) {
+                const int mk = min(m - k, 32 * ROW_SEG_MAX), sk = (mk + 31) / 32;
+                sum = warp_row_sum(sum, T + k, sk, sk, mk, codes);
+            }
+        }
+        if (lane == 0) S.sum = sum;
+    }
+    __syncthreads();
+    return S.sum;
 }
 #endif
 

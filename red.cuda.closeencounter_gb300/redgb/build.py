@@ -33,6 +33,7 @@ UNITS = {
     "small_step.cu": ["-fmad=false"],
     "gravity_mixed.cu": [],
     "swarm_step.cu": [],
+    "swarm_fp64.cu": ["-fmad=false"],
     "ensemble.cu": ["-fmad=false"],
     "mlp.cu": [],
     "noalloc.cu": ["-fmad=false"],
