@@ -20,6 +20,7 @@
 // The row-serial kernel (thread per sink) serves blocks with few sources per sink
 // (planetesimals x 3 massive bodies).  Sources are staged through shared memory in both.
 #include <atomic>
+#include <type_traits>
 #include <string>
 
 #include "../../include/redgb.h"
@@ -193,30 +194,52 @@ __global__ void star_distance(const double* __restrict__ x, const double* __rest
 // Row path: rows whose sums need every bit of their terms -- blocks with a handful of sinks and
 // many sources (the star and giants of a planetesimal disk), and the rows gravity_cert.cu leaves
 // over.  One CTA per row: eight warps compute the exact terms of a chunk of sources into shared
-// memory while three others, one per component, add the chunk before it in ascending source
-// order (warp_row_sum, row_sum.h).
+// memory while three groups of two, one per component, add the chunk before it in ascending source
+// order (group_row_sum, row_sum.h).
 //
-// Bound: a chunk of 1152 pairs is 36 warps x 12 FP64 operations x 16 cycles of the SM's FP64 pipe
-// (6.9 k cycles), its sums 4-12 k cycles of latency beside them; the serial additions they replace
-// took 71 cycles per term.
+// Bound: a chunk's 1152 pairs, 36 warps x (12 FP64 operations x 16 cycles of the SM's FP64 pipe and
+// the integer square root and division), about 12 k cycles; the sums take as long beside them,
+// also where they hover (one warp a component: up to 30 k cycles a chunk for a coplanar system's z
+// row).
+//
+// A listed row (LIST) has other rows beside it on its SM, three CTAs with a summing warp per component
+// (warp_row_sum): a force evaluation of the dense ring, 11 000 listed rows, 131.5 ms, with the two
+// CTAs that the groups leave room for 135.2 ms.  Few rows have an SM each: 64 disks in FP64 131 ms
+// with single warps, 117 ms with groups.
 constexpr int ROW_TERM_WARPS = 8;
-constexpr int ROW_WARPS = 3 + ROW_TERM_WARPS;
-constexpr int ROW_CHUNK = 32 * ROW_SEG_MAX;
-constexpr int ROW_PITCH = 32 * (ROW_SEG_MAX | 1);
+constexpr int ROW_CHUNK = 1152;
+static_assert(ROW_CHUNK >= 32 * ROW_SEG_MAX, "codes of a chunk");
 
+template <bool LIST>
+struct RowShape {
+    static constexpr int SUM_WARPS = LIST ? 1 : 2;  // per component
+    static constexpr int WARPS = 3 * SUM_WARPS + ROW_TERM_WARPS;
+    static constexpr int CTAS = LIST ? 3 : 2;  // per SM
+    static constexpr int LANES = 32 * SUM_WARPS;
+    static constexpr int PITCH = LANES * (ROW_CHUNK / LANES | 1);
+};
+
+struct NoRules {};
+template <bool LIST>
 struct RowSmem {
-    double term[2][3][ROW_PITCH];
-    uint32_t codes[3][32 * ROW_SEG_MAX];
+    double term[2][3][RowShape<LIST>::PITCH];
+    uint32_t codes[3][ROW_CHUNK];
+    std::conditional_t<LIST, NoRules, GroupRowSmem<640, RowShape<LIST>::SUM_WARPS>> sum[3];
 };
 
 // LIST: the rows *n_list of `list` (part: components to add), without event tests
 template <bool LIST>
-__global__ void __launch_bounds__(32 * ROW_WARPS) grav_fp64_rows(GravArgs g, const Tile* list, const unsigned int* n_list)
+__global__ void __launch_bounds__(32 * RowShape<LIST>::WARPS, RowShape<LIST>::CTAS)
+    grav_fp64_rows(GravArgs g, const Tile* list, const unsigned int* n_list)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
-    RowSmem& M = *reinterpret_cast<RowSmem*>(row_smem);
+    using Shape = RowShape<LIST>;
+    constexpr int LANES = Shape::LANES;
+    RowSmem<LIST>& M = *reinterpret_cast<RowSmem<LIST>*>(row_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_rows = LIST ? (int)*n_list : g.n_tiles;
+    const int comp = warp / Shape::SUM_WARPS;  // of a sum warp: 0, 1, 2
+    [[maybe_unused]] const RowGroup grp{1 + min(comp, 3), LANES, (int)threadIdx.x - LANES * comp};
     for (int row = blockIdx.x; row < n_rows; row += gridDim.x) {
         const Tile tile = LIST ? list[row] : g.tiles[row];
         if (g.sys_active && !g.sys_active[tile.sys]) continue;
@@ -228,11 +251,12 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) grav_fp64_rows(GravArgs g, con
         double acc = 0.0;
         const int n = tile.src_end - tile.src_begin;
         const int chunks = (n + ROW_CHUNK - 1) / ROW_CHUNK;
+        const bool adds = comp < 3 && (comps >> comp & 1);
         for (int c = 0; c <= chunks; c++) {
-            if (c < chunks && (c == 0 || warp >= 3)) {  // terms of chunk c (the first one: by every warp)
+            if (c < chunks && (c == 0 || comp >= 3)) {  // terms of chunk c (the first one: by every warp)
                 const int q0 = c * ROW_CHUNK, m = min(ROW_CHUNK, n - q0);
-                const int seg = (m + 31) / 32, pitch = seg | 1;
-                const int w0 = c == 0 ? 0 : 3, nw = ROW_WARPS - w0;
+                const int seg = (m + LANES - 1) / LANES, pitch = seg | 1;
+                const int w0 = c == 0 ? 0 : 3 * Shape::SUM_WARPS, nw = Shape::WARPS - w0;
                 for (int q = (warp - w0) * 32 + lane; q < m; q += 32 * nw) {
                     const int j = tile.src_begin + q0 + q;
                     const double xj = g.px[j], yj = g.py[j], zj = g.pz[j], mj = g.mass[j];
@@ -246,14 +270,18 @@ __global__ void __launch_bounds__(32 * ROW_WARPS) grav_fp64_rows(GravArgs g, con
                     M.term[c & 1][2][at] = o.tz;
                 }
             }
-            if (c > 0 && warp < 3 && (comps >> warp & 1)) {
+            if (c > 0 && adds) {
                 const int m = min(ROW_CHUNK, n - (c - 1) * ROW_CHUNK);
-                const int seg = (m + 31) / 32;
-                acc = warp_row_sum(acc, M.term[(c - 1) & 1][warp], seg, seg | 1, m, M.codes[warp]);
+                const int seg = (m + LANES - 1) / LANES;
+                const double* const T = M.term[(c - 1) & 1][comp];
+                if constexpr (LIST)
+                    acc = warp_row_sum(acc, T, seg, seg | 1, m, M.codes[comp]);
+                else
+                    acc = group_row_sum(grp, acc, T, seg, seg | 1, m, M.codes[comp], M.sum[comp]);
             }
             __syncthreads();
         }
-        if (warp < 3 && lane == 0 && (comps >> warp & 1)) (warp == 0 ? g.ax : warp == 1 ? g.ay : g.az)[i] = acc;
+        if (adds && (int)threadIdx.x == LANES * comp) (comp == 0 ? g.ax : comp == 1 ? g.ay : g.az)[i] = acc;
     }
 }
 
@@ -328,9 +356,10 @@ static int row_attributes()
     int dev = 0;
     RG_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        const int smem = (int)sizeof(RowSmem);
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(RowSmem<true>)));
+        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)sizeof(RowSmem<false>)));
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
     return 0;
@@ -340,7 +369,7 @@ int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
     if (const int rc = row_attributes()) return rc;
-    grav_fp64_rows<false><<<g.n_tiles, 32 * ROW_WARPS, sizeof(RowSmem), st>>>(g, nullptr, nullptr);
+    grav_fp64_rows<false><<<g.n_tiles, 32 * RowShape<false>::WARPS, sizeof(RowSmem<false>), st>>>(g, nullptr, nullptr);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }
@@ -348,8 +377,9 @@ int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st)
 int launch_grav_fp64_list(const GravArgs& g, const CertRows& cr, cudaStream_t st)
 {
     if (const int rc = row_attributes()) return rc;
-    // as many CTAs as are resident (three per SM); the list's length is known on the device
-    grav_fp64_rows<true><<<3 * NUM_SMS_HINT, 32 * ROW_WARPS, sizeof(RowSmem), st>>>(g, cr.list, cr.n_list);
+    // as many CTAs as are resident; the list's length is known on the device
+    using Shape = RowShape<true>;
+    grav_fp64_rows<true><<<Shape::CTAS * NUM_SMS_HINT, 32 * Shape::WARPS, sizeof(RowSmem<true>), st>>>(g, cr.list, cr.n_list);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

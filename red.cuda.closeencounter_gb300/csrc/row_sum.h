@@ -339,46 +339,61 @@ __device__ __forceinline__ double warp_row_sum(double acc, const double* T, int 
     return __longlong_as_double((long long)__shfl_sync(ALL, (unsigned long long)mine, 31));
 }
 
-// The same sum by all W warps of a CTA (blockDim.x = 32 W), each lane one of 32 W segments: the
-// lanes' passes get as many times shorter, the codes are still applied in order, by the first
-// warp, one after the other from one list.  Terms T[0 .. m) in shared memory, m <= 32 W
-// ROW_SEG_MAX; every thread of the CTA calls this and gets the sum.  A slow lane is added again
-// from its true start when its turn comes; a row with too many of them, or with offsets out of
+// The same sum by a group of W warps (a CTA, or warps with a named barrier of their own), each lane one
+// of 32 W segments: the lanes' passes get as many times shorter, the codes are still applied in
+// order, by the first warp, one after the other from one list.  A slow lane is added again from its
+// true start when its turn comes; a row with too many of them or of codes, or with offsets out of
 // range, is summed by the first warp alone.
 // Measured: a hovering row of 1027 terms (some 250 codes) 15.5 k cycles of eight warps,
 // warp_row_sum 28 k.
-constexpr int ROW_RULES = 1024;  // most codes of a row that are applied
-constexpr int ROW_HARD = 8;      // most lanes of a row that are added again
-struct CtaRowSmem {
-    rs::RowRule rule[ROW_RULES];
+constexpr int ROW_HARD = 8;  // most lanes of a row that are added again
+struct RowGroup {
+    int id, threads, me;  // named barrier, its threads, this one of them
+    __device__ void sync() const { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+    __device__ bool any(bool p) const
+    {
+        int r;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.s32 p, %1, 0;\n\tbar.red.or.pred q, %2, %3, p;\n\tselp.s32 %0, 1, 0, q;\n\t}"
+                     : "=r"(r)
+                     : "r"((int)p), "r"(id), "r"(threads)
+                     : "memory");
+        return r != 0;
+    }
+};
+template <int RULES, int WARPS>  // RULES: most codes of a row that are applied
+struct GroupRowSmem {
+    rs::RowRule rule[RULES];
     struct {
         int lane, rule, in;  // the lane, its place among the rules, the offset's change since the lane with codes before
         unsigned long long before, end;
     } hard[ROW_HARD];
-    int P[32 * ROW_CTA_WARPS];  // of the lanes with codes
-    int top[ROW_CTA_WARPS];
-    long long units[ROW_CTA_WARPS];
-    unsigned long long end[ROW_CTA_WARPS], last;
-    int diff[ROW_CTA_WARPS], count[ROW_CTA_WARPS], coded[ROW_CTA_WARPS];
+    int P[32 * WARPS];  // of the lanes with codes
+    int top[WARPS];
+    long long units[WARPS];
+    unsigned long long end[WARPS], last;
+    int diff[WARPS], count[WARPS], coded[WARPS];
     int last_in;
     double sum;
 };
 
-// codes: max(m, 32 ROW_SEG_MAX) entries at least
-__device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* codes, CtaRowSmem& S)
+// acc + T_0 + ... + T_{m-1}: term e is at T[e / seg * pitch + e % seg], seg <= ROW_SEG_MAX, m <= 32 W
+// seg; every thread of the group calls this and gets the sum.  codes: max(m, 32 ROW_SEG_MAX)
+// entries of shared memory at least.
+template <int RULES, int WARPS>
+__device__ __forceinline__ double group_row_sum(const RowGroup& grp, double acc, const double* T, int seg, int pitch,
+                                                int m, uint32_t* codes, GroupRowSmem<RULES, WARPS>& S)
 {
     constexpr unsigned ALL = 0xffffffffu;
-    const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, me = threadIdx.x;
-    const int seg = (m + 32 * W - 1) / (32 * W);
+    const int me = grp.me, W = grp.threads >> 5, warp = me >> 5, lane = me & 31;
     const int n = max(0, min(seg, m - me * seg));
-    const double* const t = T + me * seg;
-    int top = 0;
+    const double* const t = T + me * pitch;
+    int top = (int)((uint32_t)(xf::dbits(acc) >> 52) & 0x7ffu);
     for (int k = 0; k < n; k++) top = max(top, (int)((uint32_t)(xf::dbits(t[k]) >> 52) & 0x7ffu));
     top = __reduce_max_sync(ALL, top);
     if (lane == 0) S.top[warp] = top;
-    __syncthreads();
+    grp.sync();
     for (int w = 0; w < W; w++) top = max(top, S.top[w]);
-    long long u = 0;
+    long long u = me == 0 ? rs::row_units(xf::dbits(acc), top) : 0;
     for (int k = 0; k < n; k++) u += rs::row_units(xf::dbits(t[k]), top);
     const long long own = u;
 #pragma unroll
@@ -387,10 +402,10 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
         if (lane >= off) u += o;
     }
     if (lane == 31) S.units[warp] = u;
-    __syncthreads();
+    grp.sync();
     long long base = u - own;
     for (int w = 0; w < warp; w++) base += S.units[w];
-    double a = __longlong_as_double((long long)rs::row_from_units(base, top));  // (the first lane: 0.0)
+    double a = me == 0 ? acc : __longlong_as_double((long long)rs::row_from_units(base, top));
     const uint64_t guess = xf::dbits(a);
     bool hard = rs::near_edge(guess);
     int nc = 0;
@@ -404,8 +419,8 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
     for (int q = 0; q < nc; q++) code[q] = rs::row_code(code[q], xf::dbits(t[code[q] >> 13 & 63u]));
     const uint64_t end = xf::dbits(a);
     if (lane == 31) S.end[warp] = end;
-    if (me == (int)blockDim.x - 1) S.last = end;
-    __syncthreads();
+    if (me == grp.threads - 1) S.last = end;
+    grp.sync();
     uint64_t before = __shfl_up_sync(ALL, (unsigned long long)end, 1);
     if (lane == 0 && warp > 0) before = S.end[warp - 1];
     int d = 0;
@@ -414,7 +429,7 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
         loose = false;
         d = 0;
     }
-    if (!__syncthreads_or(loose || d != 0)) return __longlong_as_double((long long)S.last);
+    if (!grp.any(loose || d != 0)) return __longlong_as_double((long long)S.last);
     // the lanes' offsets if none had codes, and where a lane's codes stand among all (the first
     // lane's change nothing: its offset is 0)
     const bool again = me > 0 && (hard || loose), has = me > 0 && (again || nc > 0);
@@ -434,7 +449,7 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
         S.count[warp] = at;
         S.coded[warp] = order;
     }
-    __syncthreads();
+    grp.sync();
     int total = 0;
     for (int w = 0; w < W; w++) {
         if (w < warp) {
@@ -446,9 +461,9 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
     }
     const int n_hard = total >> 20, n_rule = total & 0xfffff;
     if (has) S.P[order - 1] = P;
-    bool slow = __syncthreads_or(n_rule > ROW_RULES || n_hard > ROW_HARD);
+    bool slow = grp.any(n_rule > RULES || n_hard > ROW_HARD);
     const int since = P - (order - (int)has > 0 ? S.P[order - (int)has - 1] : 0);
-    if (me == (int)blockDim.x - 1) S.last_in = has ? 0 : since;
+    if (me == grp.threads - 1) S.last_in = has ? 0 : since;
     bool fit = true;
     if (!slow && has) {
         const int first = (at & 0xfffff) - mine;
@@ -464,7 +479,7 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
         }
     }
     constexpr int LIM = 1 << 29;
-    slow = __syncthreads_or(slow || !fit);
+    slow = grp.any(slow || !fit);
     if (warp == 0) {
         int off = 0, most = slow ? LIM : 0;
         uint64_t tend = 0;  // the true end of the last lane added again
@@ -477,24 +492,29 @@ __device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* 
             const auto& h = S.hard[k];
             const bool follows = k > 0 && S.hard[k - 1].lane == h.lane - 1;
             double b = __longlong_as_double((long long)(follows ? tend : rs::row_shift(h.before, off + h.in)));
-            for (int e = h.lane * seg; e < min(m, h.lane * seg + seg); e++) b = __dadd_rn(b, T[e]);
+            for (int e = 0; e < min(seg, m - h.lane * seg); e++) b = __dadd_rn(b, T[h.lane * pitch + e]);
             tend = xf::dbits(b);
             if (!rs::row_diff(tend, h.end, &off, LIM)) most = LIM;
             q = to + 1;
         }
-        double sum = 0.0;
-        if (most < LIM) {
+        double sum = acc;
+        if (most < LIM)
             sum = __longlong_as_double((long long)rs::row_shift(S.last, off + S.last_in));
-        } else {  // (the codes' space is free: they are not used)
-            for (int k = 0; k < m; k += 32 * ROW_SEG_MAX) {
-                const int mk = min(m - k, 32 * ROW_SEG_MAX), sk = (mk + 31) / 32;
-                sum = warp_row_sum(sum, T + k, sk, sk, mk, codes);
-            }
-        }
+        else  // (the codes' space is free: they are not used)
+            for (int w = 0; w < W && w * 32 * seg < m; w++)
+                sum = warp_row_sum(sum, T + w * 32 * pitch, seg, pitch, min(m - w * 32 * seg, 32 * seg), codes);
         if (lane == 0) S.sum = sum;
     }
-    __syncthreads();
+    grp.sync();
     return S.sum;
+}
+
+// by a whole CTA of at most ROW_CTA_WARPS warps, from zero, the terms one after the other
+using CtaRowSmem = GroupRowSmem<1024, ROW_CTA_WARPS>;
+__device__ __forceinline__ double cta_row_sum(const double* T, int m, uint32_t* codes, CtaRowSmem& S)
+{
+    const int seg = (m + (int)blockDim.x - 1) / (int)blockDim.x;
+    return group_row_sum(RowGroup{0, (int)blockDim.x, (int)threadIdx.x}, 0.0, T, seg, seg, m, codes, S);
 }
 #endif
 

@@ -82,4 +82,4 @@ def test_cta_row_sum(tmp_path):
     r = subprocess.run([exe, "4000"], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
     rows = re.findall(r"family \d warps \d+ rows \d+ bad (\d+)", r.stdout)
-    assert len(rows) == 10 and all(int(b) == 0 for b in rows), r.stdout
+    assert len(rows) == 15 and all(int(b) == 0 for b in rows), r.stdout
