@@ -67,12 +67,16 @@ constexpr int64_t UNCERTAIN = 1ll << 36;  // terms this large are rarely certain
 constexpr float MIN_R2 = 8.3e-25f;    // 2^-80: closer pairs (and the sink itself) are taken exactly
 constexpr float MIN_MASS = 5.3e-23f;  // 2^-74: lighter masses have no exact split
 constexpr float FAR = 1.0e15f;        // beyond the splits' range
-constexpr int CERT_WARPS = 2;         // independent warps per CTA
+constexpr int CERT_WARPS = 1;         // independent warps per CTA (2: 1.9 % slower at 16 385 and 131 074 bodies)
 
-// per warp: SW sinks, 32 / SW lanes on each (2, 4 and 8 sinks per warp: 3.0, 2.5 and 2.8 ms per
-// evaluation of 16 385 bodies)
-constexpr int SW = 4;
+// per warp: SW sinks, 32 / SW lanes on each.  Four where the sinks fill the chip with warps (2, 4 and
+// 8 sinks per warp: 3.0, 2.5 and 2.8 ms per evaluation of 16 385 bodies when this was first
+// measured, 2.47 against 2.38 ms now; 916 against 871 us for 9001), two below ten such warps an SM,
+// where twice the warps hide more latency (2001 / 2999 / 4501 bodies: 153 / 212 / 343 us, with four
+// 180 / 236 / 369 us; 6001 bodies: the same).
+constexpr int CERT_FULL = 10;  // warps an SM
 
+template <int SW>
 struct alignas(16) CertSmem {  // rows are read and copied to 16 bytes at a time
     static constexpr int NQ = 32 / SW;       // slices
     static constexpr int SLICE = 32;         // sources of a lane per epoch: one flag bit each
@@ -439,11 +443,11 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 // has few certain terms.  Once more than an eighth of an epoch's pairs are uncertain in it, or it
 // has left its binade in four epochs, the sink goes to a list of rows, the component is dropped
 // here, and grav_fp64_rows adds it from exact terms.
-template <bool SCREEN>
+template <int SW, bool SCREEN>
 __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     grav_fp64_cert(GravArgs g, CertRows cr)
 {
-    using Sm = CertSmem;
+    using Sm = CertSmem<SW>;
     static_assert(sizeof(Sm) % 16 == 0 && Sm::PITCH % 4 == 0 && HEAD % 4 == 0, "16-byte copies");
     constexpr int NQ = Sm::NQ, PITCH = Sm::PITCH, SLICE = Sm::SLICE, PART = Sm::PART, EPOCH = SLICE * NQ;
     constexpr unsigned ALL = 0xffffffffu;
@@ -785,23 +789,23 @@ int launch_cert_prep(const GravArgs& g, const int* sys_base, const int* sys_n, i
 int launch_grav_fp64_cert(const GravArgs& g, const CertRows& cr, int S, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
-    // eight CTAs per SM need more than the default shared-memory carve-out: a per-device attribute of each
+    // the CTAs of an SM need more than the default shared-memory carve-out: a per-device attribute of each
     // kernel, set once per device (setting it again from another thread is harmless)
     static std::atomic<bool> attr_set[64];
     int dev = 0;
     RG_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_cert<true>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           cudaSharedmemCarveoutMaxShared));
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_cert<false>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                           cudaSharedmemCarveoutMaxShared));
+        for (auto kernel : {grav_fp64_cert<2, true>, grav_fp64_cert<2, false>, grav_fp64_cert<4, true>, grav_fp64_cert<4, false>})
+            RG_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                               cudaSharedmemCarveoutMaxShared));
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
-    const dim3 grid(g.n_tiles, (S + SW * CERT_WARPS - 1) / (SW * CERT_WARPS));
-    if (g.record || g.hill)
-        grav_fp64_cert<true><<<grid, 32 * CERT_WARPS, 0, st>>>(g, cr);
-    else
-        grav_fp64_cert<false><<<grid, 32 * CERT_WARPS, 0, st>>>(g, cr);
+    const bool few = (long long)g.n_tiles * S <= 4LL * CERT_FULL * NUM_SMS_HINT;
+    const int per_cta = (few ? 2 : 4) * CERT_WARPS;
+    const dim3 grid(g.n_tiles, (S + per_cta - 1) / per_cta);
+    auto kernel = few ? (g.record || g.hill ? grav_fp64_cert<2, true> : grav_fp64_cert<2, false>)
+                      : (g.record || g.hill ? grav_fp64_cert<4, true> : grav_fp64_cert<4, false>);
+    kernel<<<grid, 32 * CERT_WARPS, 0, st>>>(g, cr);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }
