@@ -100,9 +100,9 @@ constexpr int FEW_SINKS_MAX = 8;  // sinks per few-sink tile (mixed mode)
 int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st);
 // blocks of up to this many (sink, source) pairs go row by row, larger ones to gravity_cert.cu: a
 // row's latency is a few microseconds and its pairs cost five times as much.  Self-interacting
-// blocks of 400 / 1000 / 1500 / 2000 / 3000 bodies on GB300: rows 22 / 58 / 110 / 179 / 363 us,
-// gravity_cert.cu 60 / 98 / 140 / 169 / 228 us.
-constexpr int64_t FP64_ROW_PAIRS = 3200000;
+// blocks of 400 / 1000 / 1300 / 1500 / 1700 / 2000 bodies on GB300: rows 18 / 62 / 93 / 110 / 146 /
+// 195 us, gravity_cert.cu 48 / 88 / 99 / 110 / 124 / 149 us.
+constexpr int64_t FP64_ROW_PAIRS = 2250000;
 // mixed precision (gravity_mixed.cu): positions split into FP32 (hi, lo) once per evaluation
 struct SplitPos;
 constexpr int MIXED_SINKS_PER_TILE = 128;
