@@ -144,54 +144,71 @@ __device__ __forceinline__ bool mine(const EnsEventArgs& a, int s, const DevEven
 }  // namespace
 
 // ------------------------------------------------------------------- Hill-sphere records
-constexpr int HILL_LOCAL = 48;  // a disk's records gathered in one pass (more: repeated scans)
+constexpr int HILL_LOCAL = 128;  // a disk's records gathered in one pass (more: repeated scans)
+
+__device__ void hill_event(const EnsEventArgs& a, int s, int b, const DevEvent& d)
+{
+    rg_event_t* x = log_slot(a, s);
+    if (!x) return;
+    x->event_name = RG_EVENT_CLOSE_ENCOUNTER;
+    x->t = d.t;  // the step start, where the pair was found inside the sphere
+    x->d = d.d;
+    x->id1 = a.id[d.i];
+    x->id2 = a.id[d.j];
+    x->idx1 = d.i - b;
+    x->idx2 = d.j - b;
+    x->p1 = a.prm[d.i];
+    x->p2 = a.prm[d.j];
+    x->r1 = rg_vec_t{d.ri[0], d.ri[1], d.ri[2], 0.0};
+    x->v1 = rg_vec_t{d.vi[0], d.vi[1], d.vi[2], 0.0};
+    x->r2 = rg_vec_t{d.rj[0], d.rj[1], d.rj[2], 0.0};
+    x->v2 = rg_vec_t{d.vj[0], d.vj[1], d.vj[2], 0.0};
+}
+
+__device__ __forceinline__ bool was_inside(const long long* prev, int n_prev, long long key)
+{
+    bool seen = false;
+    for (int q = 0; q < n_prev && !seen; q++) seen = prev[q] == key;
+    return seen;
+}
 
 __device__ void log_hill(const EnsEventArgs& a, int s, int b, const DevEvent& d, const long long* prev, int n_prev,
                          long long* next, int& n_next)
 {
     const long long key = pair_key(a.id[d.i], a.id[d.j]);
-    bool seen = false;
-    for (int q = 0; q < n_prev && !seen; q++) seen = prev[q] == key;
-    if (!seen) {
-        rg_event_t* x = log_slot(a, s);
-        if (x) {
-            x->event_name = RG_EVENT_CLOSE_ENCOUNTER;
-            x->t = d.t;  // the step start, where the pair was found inside the sphere
-            x->d = d.d;
-            x->id1 = a.id[d.i];
-            x->id2 = a.id[d.j];
-            x->idx1 = d.i - b;
-            x->idx2 = d.j - b;
-            x->p1 = a.prm[d.i];
-            x->p2 = a.prm[d.j];
-            x->r1 = rg_vec_t{d.ri[0], d.ri[1], d.ri[2], 0.0};
-            x->v1 = rg_vec_t{d.vi[0], d.vi[1], d.vi[2], 0.0};
-            x->r2 = rg_vec_t{d.rj[0], d.rj[1], d.rj[2], 0.0};
-            x->v2 = rg_vec_t{d.vj[0], d.vj[1], d.vj[2], 0.0};
-        }
-    }
+    if (!was_inside(prev, n_prev, key)) hill_event(a, s, b, d);
     if (n_next < a.hill_set_cap)
         next[n_next++] = key;
     else
         atomicOr(a.flags, ENS_FLAG_HILL_SET);
 }
 
-// one CTA per disk: its threads scan the step start's Hill records together and gather the
-// disk's (at most HILL_LOCAL of them; a disk with more repeats the scan for the rest, one
-// record at a time), then one thread logs them in (sink, source) order
-constexpr int HILL_THREADS = 64;
+// one CTA per disk: its threads scan the step start's Hill records together and gather the disk's
+// (at most HILL_LOCAL of them; a disk with more repeats the scan for the rest, one record at a
+// time), put them in (sink, source) order and look them up among the last step's pairs, a record a
+// thread; one thread then logs the new ones in order.  All latency: with one thread sorting and
+// looking up, 106 us for 256 disks; this way 42 us.
+constexpr int HILL_THREADS = 256;
 
 __global__ void __launch_bounds__(HILL_THREADS) ens_hill_kernel(EnsEventArgs a)
 {
-    const int s = blockIdx.x;
+    const int s = blockIdx.x, t = threadIdx.x;
     if (!a.active_f0[s]) return;  // uniform over the CTA
-    __shared__ long long key[HILL_LOCAL];
-    __shared__ unsigned int idx[HILL_LOCAL];
+    __shared__ long long key[HILL_LOCAL], before[HILL_LOCAL];
+    __shared__ unsigned int idx[HILL_LOCAL], order[HILL_LOCAL];
+    __shared__ bool fresh[HILL_LOCAL];
     __shared__ int m_sh;
-    if (threadIdx.x == 0) m_sh = 0;
+    if (t == 0) m_sh = 0;
+    const int b = a.base[s];
+    const int cur = a.hill_which[s];
+    const long long* prev = a.hill_set + ((long long)s * 2 + cur) * a.hill_set_cap;
+    long long* next = a.hill_set + ((long long)s * 2 + (cur ^ 1)) * a.hill_set_cap;
+    const int n_prev = a.hill_n[s];
+    for (int q = t; q < min(n_prev, HILL_LOCAL); q += HILL_THREADS) before[q] = prev[q];
     __syncthreads();
     const unsigned int n = min(*a.hill_count, a.ev_cap);
-    for (unsigned int k = threadIdx.x; k < n; k += HILL_THREADS) {
+#pragma unroll 4
+    for (unsigned int k = t; k < n; k += HILL_THREADS) {
         const DevEvent& d = a.hill[k];
         if (d.sys != s || d.kind != 1) continue;
         const int p = atomicAdd(&m_sh, 1);
@@ -201,29 +218,29 @@ __global__ void __launch_bounds__(HILL_THREADS) ens_hill_kernel(EnsEventArgs a)
         }
     }
     __syncthreads();
-    if (threadIdx.x != 0) return;
     const int m = m_sh;
-    const int b = a.base[s];
-    const int cur = a.hill_which[s];
-    const long long* prev = a.hill_set + ((long long)s * 2 + cur) * a.hill_set_cap;
-    long long* next = a.hill_set + ((long long)s * 2 + (cur ^ 1)) * a.hill_set_cap;
-    const int n_prev = a.hill_n[s];
+    if (m <= HILL_LOCAL) {  // uniform
+        for (int q = t; q < m; q += HILL_THREADS) {  // (the keys are distinct)
+            int rank = 0;
+            for (int p = 0; p < m; p++) rank += key[p] < key[q];
+            order[rank] = idx[q];
+        }
+        __syncthreads();
+        for (int q = t; q < m; q += HILL_THREADS) {
+            const DevEvent& d = a.hill[order[q]];
+            const long long k = pair_key(a.id[d.i], a.id[d.j]);
+            fresh[q] = !was_inside(n_prev <= HILL_LOCAL ? before : prev, n_prev, k);
+            if (q < a.hill_set_cap) next[q] = k;
+        }
+        __syncthreads();
+    }
+    if (t != 0) return;
     int n_next = 0;
     if (m <= HILL_LOCAL) {
-        // the gathered records in (sink, source) order (the keys are distinct)
-        for (int q = 1; q < m; q++) {
-            const long long kk = key[q];
-            const unsigned int kx = idx[q];
-            int p = q;
-            while (p > 0 && key[p - 1] > kk) {
-                key[p] = key[p - 1];
-                idx[p] = idx[p - 1];
-                p--;
-            }
-            key[p] = kk;
-            idx[p] = kx;
-        }
-        for (int q = 0; q < m; q++) log_hill(a, s, b, a.hill[idx[q]], prev, n_prev, next, n_next);
+        for (int q = 0; q < m; q++)
+            if (fresh[q]) hill_event(a, s, b, a.hill[order[q]]);
+        n_next = min(m, a.hill_set_cap);
+        if (m > a.hill_set_cap) atomicOr(a.flags, ENS_FLAG_HILL_SET);
     } else {
         // repeatedly the smallest key above the last
         long long last = -1;
