@@ -600,10 +600,11 @@ __device__ __forceinline__ double dither_uniform(unsigned long long seed, int d,
 // one CTA per stage tile of the disks that start a step: the tile's feature partials (max |a|,
 // min (d / mutual Hill radius)^3) go to the disk's slots by atomics; the disk's last tile to
 // finish (a ticket per disk, no waiting) takes the disk's features, resets the slots for the
-// next launch, and in its first warp evaluates the network and sets the trial step.  That CTA
-// stages the network's weights in shared memory first (as float, W2 transposed so that the
-// lanes of a warp read consecutive words).
+// next launch, and in its first warp evaluates the network and sets the trial step, from the
+// weights in shared memory (as float, W2 transposed so that the lanes of a warp read consecutive
+// words).
 constexpr int PROP_THREADS = 256;
+static_assert(MLP_OFF_B1 % 8 == 0 && MLP_OFF_W2 % 8 == 0 && MLP_OFF_B2 % 8 == 0 && MLP_OFF_W3 % 8 == 0, "16-byte loads");
 
 __global__ void __launch_bounds__(PROP_THREADS) ens_propose_kernel(PropArgs a)
 {
@@ -614,10 +615,31 @@ __global__ void __launch_bounds__(PROP_THREADS) ens_propose_kernel(PropArgs a)
     __shared__ float red_am[PROP_THREADS / 32], red_h3[PROP_THREADS / 32];
     __shared__ float4 si[FEAT_MAX_SI];
     __shared__ float si_r[FEAT_MAX_SI];
-    __shared__ float sw1[MLP_HIDDEN * MLP_IN], sb1[MLP_HIDDEN], sw2t[MLP_HIDDEN * MLP_HIDDEN], sb2[MLP_HIDDEN],
+    __shared__ float sw1[MLP_HIDDEN * MLP_IN], sb1[MLP_HIDDEN], sw2t[MLP_HIDDEN * (MLP_HIDDEN + 1)], sb2[MLP_HIDDEN],
         sw3[MLP_HIDDEN];
     __shared__ int last_sh;
     __shared__ float feat_sh[2];
+    const int tiles = a.tiles_of[d];
+    // the weights travel while the features are formed (8 to a load; by the last tile's CTA, one at
+    // a time and after its features, they took a quarter of the kernel)
+    const bool use_net = a.w && !(s.cool[d] > 0 || s.n_passed[d] < 4 || !(s.ideal_last[d] > 0.0));
+    if (use_net) {
+        auto weights = [&](int off, int n, auto put) {
+            for (int k = 8 * threadIdx.x; k < n; k += 8 * PROP_THREADS) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4*>(a.w + off + k));
+                const unsigned int w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int q = 0; q < 8; q++)
+                    put(k + q, __uint_as_float(q & 1 ? w[q >> 1] & 0xffff0000u : w[q >> 1] << 16));
+            }
+        };
+        weights(MLP_OFF_W2, MLP_HIDDEN * MLP_HIDDEN,
+                [&](int k, float v) { sw2t[(k % MLP_HIDDEN) * (MLP_HIDDEN + 1) + k / MLP_HIDDEN] = v; });
+        weights(MLP_OFF_W1, MLP_HIDDEN * MLP_IN, [&](int k, float v) { sw1[k] = v; });
+        weights(MLP_OFF_B1, MLP_HIDDEN, [&](int k, float v) { sb1[k] = v; });
+        weights(MLP_OFF_B2, MLP_HIDDEN, [&](int k, float v) { sb2[k] = v; });
+        weights(MLP_OFF_W3, MLP_HIDDEN, [&](int k, float v) { sw3[k] = v; });
+    }
     float am = 0.0f, h3 = 3.0e38f;
     {
         const int b = a.base[d], ns = a.nsi[d];
@@ -647,39 +669,30 @@ __global__ void __launch_bounds__(PROP_THREADS) ens_propose_kernel(PropArgs a)
                 am = fmaxf(am, red_am[w]);
                 h3 = fminf(h3, red_h3[w]);
             }
-            // non-negative floats order as their bit patterns
-            unsigned int* r = a.red + 3 * d;
-            atomicMax(r, __float_as_uint(am));
-            atomicMin(r + 1, __float_as_uint(h3));
-            __threadfence();
-            const unsigned int done = atomicAdd(r + 2, 1u);
-            last_sh = done + 1 == (unsigned int)a.tiles_of[d];
-            if (last_sh) {
+            if (tiles == 1) {  // the disk's only tile: its features are at hand
+                last_sh = 1;
+                feat_sh[0] = am;
+                feat_sh[1] = h3;
+            } else {
+                // non-negative floats order as their bit patterns
+                unsigned int* r = a.red + 3 * d;
+                atomicMax(r, __float_as_uint(am));
+                atomicMin(r + 1, __float_as_uint(h3));
                 __threadfence();
-                feat_sh[0] = __uint_as_float(atomicExch(r, 0u));
-                feat_sh[1] = __uint_as_float(atomicExch(r + 1, FEAT_H3_NONE_BITS));
-                atomicExch(r + 2, 0u);
+                const unsigned int done = atomicAdd(r + 2, 1u);
+                last_sh = done + 1 == (unsigned int)tiles;
+                if (last_sh) {
+                    __threadfence();
+                    feat_sh[0] = __uint_as_float(atomicExch(r, 0u));
+                    feat_sh[1] = __uint_as_float(atomicExch(r + 1, FEAT_H3_NONE_BITS));
+                    atomicExch(r + 2, 0u);
+                }
             }
         }
         __syncthreads();
         if (!last_sh) return;
         am = feat_sh[0];
         h3 = feat_sh[1];
-    }
-    const bool use_net = a.w && !(s.cool[d] > 0 || s.n_passed[d] < 4 || !(s.ideal_last[d] > 0.0));
-    if (use_net) {
-        for (int k = threadIdx.x; k < MLP_HIDDEN * MLP_HIDDEN; k += blockDim.x) {
-            const int u = k / MLP_HIDDEN, v = k % MLP_HIDDEN;  // W2[u][v] -> sw2t[v][u]
-            sw2t[v * MLP_HIDDEN + u] = __bfloat162float(a.w[MLP_OFF_W2 + k]);
-        }
-        for (int k = threadIdx.x; k < MLP_HIDDEN * MLP_IN; k += blockDim.x)
-            sw1[k] = __bfloat162float(a.w[MLP_OFF_W1 + k]);
-        for (int k = threadIdx.x; k < MLP_HIDDEN; k += blockDim.x) {
-            sb1[k] = __bfloat162float(a.w[MLP_OFF_B1 + k]);
-            sb2[k] = __bfloat162float(a.w[MLP_OFF_B2 + k]);
-            sw3[k] = __bfloat162float(a.w[MLP_OFF_W3 + k]);
-        }
-        __syncthreads();
     }
     if (threadIdx.x >= 32) return;
     const int lane = threadIdx.x & 31;
@@ -720,7 +733,7 @@ __global__ void __launch_bounds__(PROP_THREADS) ens_propose_kernel(PropArgs a)
 #pragma unroll 16
         for (int v = 0; v < 64; v++) {
             const float hv = __shfl_sync(0xffffffffu, h1[v >> 5], v & 31);
-            z = fmaf(sw2t[v * MLP_HIDDEN + u], hv, z);
+            z = fmaf(sw2t[v * (MLP_HIDDEN + 1) + u], hv, z);
         }
         h2[r] = z / (1.0f + __expf(-z));
     }
@@ -1240,8 +1253,8 @@ int upload_plans(rg_ens* e)
 }
 
 // ------------------------------------------------------------------- one attempt
-int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, int stage, const int* mask,
-                bool hill)
+GravArgs gravity_args(const rg_ens* e, const double* pos, const double* vel, double* acc, int stage, const int* mask,
+                      bool hill)
 {
     const size_t cap = (size_t)e->cap;
     GravArgs g{};
@@ -1280,6 +1293,13 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
     g.sys_attempt = e->d_attempt;
     g.sys_f0 = e->d_nf0;
     g.sys_t = e->d_t;
+    return g;
+}
+
+int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, int stage, const int* mask,
+                bool hill)
+{
+    GravArgs g = gravity_args(e, pos, vel, acc, stage, mask, hill);
     int rc = RG_OK;
     if (hill) {
         // distance from each disk's body 0 (the per-body base is the tile's base: use a
@@ -1472,6 +1492,46 @@ int launch_stage(rg_ens* e, int form, int nterm, const int* stages, const double
     return RG_OK;
 }
 
+// stage r's sums and forces in one kernel, where every disk is in symmetric segments
+bool stage_sym_fits(const rg_ens* e)
+{
+    if (e->gravity_mode != RG_GRAVITY_MIXED || e->profiling || e->plan[1].size() != 1) return false;
+    const auto& gr = e->plan[1][0];
+    if (gr.kind != GROUP_DF_SYM || gr.max_src > STAGE_SYM_HEAVY) return false;
+    for (int s = 0; s < e->n_sys; s++)
+        if (e->ntot[s] != e->n_massive(s) || e->n_massive(s) <= e->n_si(s)) return false;
+    return true;
+}
+
+int launch_stage_sym(rg_ens* e, int r)
+{
+    const size_t cap = (size_t)e->cap;
+    const auto& gr = e->plan[1][0];
+    StageSymArgs a{};
+    a.g = gravity_args(e, nullptr, nullptr, e->d_k[r] + 3 * cap, r, e->d_active, false);
+    a.g.tiles = e->d_tiles + gr.off;
+    a.g.n_tiles = gr.n;
+    a.y = e->d_y;
+    for (int q = 0; q < rk8_nterm[r]; q++) {
+        a.k[q] = e->d_k[rk8_stage[r][q]];
+        a.c[q] = rk8_a[rk8_aidx[r][q]];
+    }
+    a.dt = e->d_dt_try;
+    a.vel = e->d_k[r];
+    a.stride = e->cap;
+    a.cta_seg = e->d_sym_cta;
+    a.tile_row0 = e->d_few_row0 + gr.off;
+    a.partial = e->d_terms;
+    a.rows = e->few_rows;
+    a.pitch = e->few_pitch;
+    a.row_sink = e->d_row_sink;
+    a.row_nparts = e->d_row_nparts;
+    a.ticket = e->d_sym_ticket;
+    a.mass_f2 = e->d_mass_f2;
+    e->n_kernels++;
+    return launch_ens_stage_sym(a, rk8_nterm[r], (int)e->sym_cta.size() - 1, e->st);
+}
+
 EnsEventArgs event_args(rg_ens* e)
 {
     EnsEventArgs a{};
@@ -1591,7 +1651,12 @@ int record_attempt(rg_ens* e, bool in_graph)
         e->n_kernels++;
     }
     prof_end(e, pr);
+    const bool fused = stage_sym_fits(e);
     for (int r = 1; r <= 12 && !rc; r++) {
+        if (fused) {
+            rc = launch_stage_sym(e, r);
+            continue;
+        }
         double a[9];
         for (int q = 0; q < rk8_nterm[r]; q++) a[q] = rk8_a[rk8_aidx[r][q]];
         pr = prof_begin(e, 1);

@@ -152,6 +152,29 @@ int launch_grav_df_sym(const GravArgs& g, const int* cta_seg, int n_cta, const v
                        const int* row_nparts, unsigned int* ticket, cudaStream_t st,
                        const float2* mass_f2 = nullptr);
 
+// one stage of the ensemble's mixed form, stage sums and symmetric evaluation (ens_stage.cu): every
+// disk in symmetric segments, at most STAGE_SYM_HEAVY heavy bodies each, no test particles
+constexpr int STAGE_SYM_HEAVY = 3;
+struct StageSymArgs {
+    GravArgs g;  // (its positions and velocities are not read)
+    const double* y;        // 6 rows
+    const double* k[MAXT];  // stage vectors, double-float pairs
+    double c[MAXT];
+    const double* dt;       // per disk
+    double* vel;            // the next stage vector's velocity rows
+    int stride;
+    const int* cta_seg;     // as in launch_grav_df_sym
+    const int* tile_row0;
+    double* partial;
+    int rows;
+    long long pitch;
+    const int* row_sink;
+    const int* row_nparts;
+    unsigned int* ticket;
+    const float2* mass_f2;
+};
+int launch_ens_stage_sym(const StageSymArgs& a, int nterm, int n_cta, cudaStream_t st);
+
 int launch_star_distance(const double* x, const double* y, const double* z, const int* base_of, int n, double* rho,
                          cudaStream_t st);
 

@@ -35,6 +35,7 @@ UNITS = {
     "swarm_step.cu": [],
     "swarm_fp64.cu": ["-fmad=false"],
     "ensemble.cu": ["-fmad=false"],
+    "ens_stage.cu": [],
     "mlp.cu": [],
     "noalloc.cu": ["-fmad=false"],
     "ens_events.cu": ["-fmad=false"],
