@@ -11,17 +11,16 @@
 // bounds this file.  The square root and the division of each pair term, about half of its
 // FP64 instructions in hardware form, are computed exactly (correctly rounded, the same
 // bits) with integer arithmetic on the other pipes (exact_fp64.h); the FP64 pipe keeps the
-// 15 subtractions, multiplications and additions.  The serial sum is only 3 FP64 adds per
-// pair; the pair terms do not depend on the order.  The pair-parallel
-// kernel therefore lets all 256 threads of a CTA compute the S x J pair terms of a tile
-// (S sinks x J sources) into shared memory, and 3 S threads then add them in source
-// order.  That keeps every SM's FP64 pipe busy however few sinks a block has (3 sinks x
-// 1027 sources in the planetesimal disk), which thread-per-sink scheduling cannot.
-// The row-serial kernel (thread per sink) serves blocks with few sources per sink
-// (planetesimals x 3 massive bodies).  Sources are staged through shared memory in both.
+// additions and multiplications.  The pair terms do not depend on the order, so they are formed
+// side by side, and the sums are added in ascending j: a CTA per row (grav_fp64_rows, the sum by
+// segments, row_sum.h) for rows of many sources in blocks of few pairs, and for the rows that
+// gravity_cert.cu, which takes the large blocks, leaves over; the row-serial kernel (thread per
+// sink) for blocks with few sources per sink (planetesimals x 3 massive bodies); and the
+// pair-parallel kernel (S x J terms into shared memory, 3 S threads add them) for the
+// astrocentric frame.
 #include <atomic>
-#include <type_traits>
 #include <string>
+#include <type_traits>
 
 #include "../../include/redgb.h"
 #include "common.cuh"
@@ -45,8 +44,8 @@ int set_error(int code, const std::string& msg);
 
 // S sinks x STRIDE threads per CTA, four pair terms per thread and tile (J = 4 STRIDE sources).
 // S sets the number of CTAs, ceil(sinks / S): the tuner picks the S whose grid fills the last
-// wave of resident CTAs best (16 385 sinks at S = 36: 456 CTAs, exactly three per SM of a
-// 152-SM GB300), since every CTA of a block runs the same sources and so takes the same time.
+// wave of resident CTAs best, since every CTA of a block runs the same sources and so takes the
+// same time.  Launched for the astrocentric frame.
 template <int S, int STRIDE, bool ASTRO>
 __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pairpar(GravArgs g)
 {

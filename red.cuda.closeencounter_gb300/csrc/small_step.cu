@@ -8,8 +8,8 @@
 // terms stay in shared memory; pairs, sums and state elements are each dealt out densely over
 // the threads, because a warp's FP64 instruction costs its SM sub-partition 64 cycles however
 // few lanes are active (a warp per body took 75 us per attempt of nine bodies, this form
-// 38; a step 281 us before, 45 now, with the host's launch and wait).  The arithmetic is the other kernels': pair_term, the sums in ascending source
-// order, the stage sums of stages.cu.
+// 38; a step 281 us before, 45 now, with the host's launch and wait).  The arithmetic is the
+// other kernels': pair_term, the sums in ascending source order, the stage sums of stages.cu.
 #include <algorithm>
 #include <atomic>
 
