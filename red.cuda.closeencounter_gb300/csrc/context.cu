@@ -694,7 +694,7 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
             c->n_kernels++;
             break;
         case GROUP_FP64_ROWS:
-            rc = launch_grav_fp64_rows(g, fork_few ? c->st2 : c->st);
+            rc = launch_grav_fp64_rows(g, gr.max_src, fork_few ? c->st2 : c->st);
             c->n_kernels++;
             break;
         case GROUP_DF_ROWSEQ:

@@ -1187,6 +1187,7 @@ void build_gravity_plan(rg_ens* e)
                     gr.max_src = std::max(gr.max_src, nh);
                 } else {
                     e->few_row0.push_back(0);
+                    gr.max_src = std::max(gr.max_src, T[k].src_end - T[k].src_begin);
                 }
             }
             e->plan[mode].push_back(gr);
@@ -1367,7 +1368,7 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
             break;
         case GROUP_ROWSEQ: rc = launch_grav_fp64_rowseq(g, row_st); e->n_kernels++; break;
         case GROUP_FP64_ROWS:
-            rc = launch_grav_fp64_rows(g, e->st);
+            rc = launch_grav_fp64_rows(g, gr.max_src, e->st);
             e->n_kernels++;
             break;
         case GROUP_DF_ROWSEQ:

@@ -192,7 +192,7 @@ __global__ void star_distance(const double* __restrict__ x, const double* __rest
 // ---------------------------------------------------------------------------------------
 // Row path: rows whose sums need every bit of their terms -- blocks with a handful of sinks and
 // many sources (the star and giants of a planetesimal disk), and the rows gravity_cert.cu leaves
-// over.  One CTA per row: eight warps compute the exact terms of a chunk of sources into shared
+// over.  One CTA per row: six or eight warps compute the exact terms of a chunk of sources into shared
 // memory while three groups of two, one per component, add the chunk before it in ascending source
 // order (group_row_sum, row_sum.h).
 //
@@ -204,37 +204,41 @@ __global__ void star_distance(const double* __restrict__ x, const double* __rest
 // A listed row (LIST) has other rows beside it on its SM, three CTAs with a summing warp per component
 // (warp_row_sum): a force evaluation of the dense ring, 11 000 listed rows, 131.5 ms, with the two
 // CTAs that the groups leave room for 135.2 ms.  Few rows have an SM each: 64 disks in FP64 131 ms
-// with single warps, 117 ms with groups.
-constexpr int ROW_TERM_WARPS = 8;
+// with single warps, 117 ms with groups beside eight warps for the terms, 114 ms beside six, which
+// leave more issue slots to the sums' first warps (four: 126 ms).
+//
+// TERMS, the warps for the terms: six (self-interacting blocks of 300 / 500 / 1000 / 1480 bodies: 14.4
+// / 22.8 / 56 / 101 us, with eight 14.9 / 25.0 / 62 / 110 us), except where eight form a row's only
+// chunk at once and six do not (400 bodies: 18.3 against 20.8 us).
 constexpr int ROW_CHUNK = 1152;
 static_assert(ROW_CHUNK >= 32 * ROW_SEG_MAX, "codes of a chunk");
 
-template <bool LIST>
+template <bool LIST, int TERMS>
 struct RowShape {
     static constexpr int SUM_WARPS = LIST ? 1 : 2;  // per component
-    static constexpr int WARPS = 3 * SUM_WARPS + ROW_TERM_WARPS;
+    static constexpr int WARPS = 3 * SUM_WARPS + TERMS;  // (all of them form the first chunk's terms)
     static constexpr int CTAS = LIST ? 3 : 2;  // per SM
     static constexpr int LANES = 32 * SUM_WARPS;
     static constexpr int PITCH = LANES * (ROW_CHUNK / LANES | 1);
 };
 
 struct NoRules {};
-template <bool LIST>
+template <bool LIST, int TERMS>
 struct RowSmem {
-    double term[2][3][RowShape<LIST>::PITCH];
+    double term[2][3][RowShape<LIST, TERMS>::PITCH];
     uint32_t codes[3][ROW_CHUNK];
-    std::conditional_t<LIST, NoRules, GroupRowSmem<640, RowShape<LIST>::SUM_WARPS>> sum[3];
+    std::conditional_t<LIST, NoRules, GroupRowSmem<640, RowShape<LIST, TERMS>::SUM_WARPS>> sum[3];
 };
 
 // LIST: the rows *n_list of `list` (part: components to add), without event tests
-template <bool LIST>
-__global__ void __launch_bounds__(32 * RowShape<LIST>::WARPS, RowShape<LIST>::CTAS)
+template <bool LIST, int TERMS>
+__global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LIST, TERMS>::CTAS)
     grav_fp64_rows(GravArgs g, const Tile* list, const unsigned int* n_list)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
-    using Shape = RowShape<LIST>;
+    using Shape = RowShape<LIST, TERMS>;
     constexpr int LANES = Shape::LANES;
-    RowSmem<LIST>& M = *reinterpret_cast<RowSmem<LIST>*>(row_smem);
+    RowSmem<LIST, TERMS>& M = *reinterpret_cast<RowSmem<LIST, TERMS>*>(row_smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n_rows = LIST ? (int)*n_list : g.n_tiles;
     const int comp = warp / Shape::SUM_WARPS;  // of a sum warp: 0, 1, 2
@@ -355,20 +359,27 @@ static int row_attributes()
     int dev = 0;
     RG_CUDA_CHECK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64 || !attr_set[dev].load(std::memory_order_acquire)) {
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(RowSmem<true>)));
-        RG_CUDA_CHECK(cudaFuncSetAttribute(grav_fp64_rows<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)sizeof(RowSmem<false>)));
+        auto set = [](auto kernel, size_t bytes) {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        };
+        RG_CUDA_CHECK(set(grav_fp64_rows<true, 8>, sizeof(RowSmem<true, 8>)));
+        RG_CUDA_CHECK(set(grav_fp64_rows<false, 6>, sizeof(RowSmem<false, 6>)));
+        RG_CUDA_CHECK(set(grav_fp64_rows<false, 8>, sizeof(RowSmem<false, 8>)));
         if (dev >= 0 && dev < 64) attr_set[dev].store(true, std::memory_order_release);
     }
     return 0;
 }
 
-int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st)
+int launch_grav_fp64_rows(const GravArgs& g, int max_src, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
     if (const int rc = row_attributes()) return rc;
-    grav_fp64_rows<false><<<g.n_tiles, 32 * RowShape<false>::WARPS, sizeof(RowSmem<false>), st>>>(g, nullptr, nullptr);
+    using Six = RowShape<false, 6>;
+    using Eight = RowShape<false, 8>;
+    if (max_src > 32 * Six::WARPS && max_src <= 32 * Eight::WARPS)
+        grav_fp64_rows<false, 8><<<g.n_tiles, 32 * Eight::WARPS, sizeof(RowSmem<false, 8>), st>>>(g, nullptr, nullptr);
+    else
+        grav_fp64_rows<false, 6><<<g.n_tiles, 32 * Six::WARPS, sizeof(RowSmem<false, 6>), st>>>(g, nullptr, nullptr);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }
@@ -377,8 +388,8 @@ int launch_grav_fp64_list(const GravArgs& g, const CertRows& cr, cudaStream_t st
 {
     if (const int rc = row_attributes()) return rc;
     // as many CTAs as are resident; the list's length is known on the device
-    using Shape = RowShape<true>;
-    grav_fp64_rows<true><<<Shape::CTAS * NUM_SMS_HINT, 32 * Shape::WARPS, sizeof(RowSmem<true>), st>>>(g, cr.list, cr.n_list);
+    using Shape = RowShape<true, 8>;
+    grav_fp64_rows<true, 8><<<Shape::CTAS * NUM_SMS_HINT, 32 * Shape::WARPS, sizeof(RowSmem<true, 8>), st>>>(g, cr.list, cr.n_list);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }

@@ -97,11 +97,12 @@ int launch_astro_terms(const double* x, const double* y, const double* z, const 
 int launch_grav_fp64_rowseq(const GravArgs& g, cudaStream_t st);
 constexpr int FEW_SINKS_MAX = 8;  // sinks per few-sink tile (mixed mode)
 // FP64 rows of tiles of one sink each: exact terms added in order (gravity_fp64.cu)
-int launch_grav_fp64_rows(const GravArgs& g, cudaStream_t st);
+int launch_grav_fp64_rows(const GravArgs& g, int max_src, cudaStream_t st);  // max_src: a row's most sources
 // blocks of up to this many (sink, source) pairs go row by row, larger ones to gravity_cert.cu: a
 // row's latency is a few microseconds and its pairs cost five times as much.  Self-interacting
-// blocks of 400 / 1000 / 1300 / 1500 / 1700 / 2000 bodies on GB300: rows 18 / 62 / 93 / 110 / 146 /
-// 195 us, gravity_cert.cu 48 / 88 / 99 / 110 / 124 / 149 us.
+// blocks of 400 / 1000 / 1300 / 1480 bodies on GB300: rows 18 / 55 / 85 / 101 us, gravity_cert.cu
+// 48 / 88 / 99 / 109 us; of 1700 and 2000, before the rows' last gain of a tenth, rows 146 / 195
+// us, gravity_cert.cu 124 / 149 us.
 constexpr int64_t FP64_ROW_PAIRS = 2250000;
 // mixed precision (gravity_mixed.cu): positions split into FP32 (hi, lo) once per evaluation
 struct SplitPos;

@@ -1,5 +1,6 @@
-"""The certified FP64 gravity's two warp shapes (two sinks a warp below ten warps an SM, four above)
-and the line between it and the row kernel, against the oracle bit for bit."""
+"""The certified FP64 gravity's two warp shapes (two sinks a warp below ten warps an SM, four above),
+the row kernel's two (around rows of 384 and 448 sources) and the line between the kernels, against
+the oracle bit for bit."""
 import numpy as np
 import pytest
 
@@ -17,7 +18,7 @@ def _same(d):
         assert H.same(ag[f], ao[f]), (f, int((ag[f] != ao[f]).sum()))
 
 
-@pytest.mark.parametrize("n", [1498, 1500, 6063, 6079, 6080, 6095, 7001])
+@pytest.mark.parametrize("n", [383, 384, 447, 448, 1498, 1500, 6063, 6079, 6080, 6095, 7001])
 def test_sizes(gpulib, n):
     _same(bodies.make_disk(n_pl=n, pl_type=T.BODY_PROTOPLANET, giants=(), seed=n, m_range=(1e-9, 1e-7)))
 
