@@ -34,8 +34,8 @@ namespace redgb {
 int set_error(int code, const std::string& msg);
 
 // ---------------------------------------------------------------------------------------
-// Pair-parallel kernel: CTA = S sinks, source tiles of J = 1024 / S.  ASTRO: the
-// astrocentric frame of the reference's CPU path -- each sink starts from the star's pull
+// Pair-parallel kernel: CTA = S sinks, source tiles of J = 1024 / S, for the astrocentric frame
+// of the reference's CPU path -- each sink starts from the star's pull
 // and, for every source it interacts with, adds the direct term and then subtracts the
 // source's indirect term (pp_disk.cu:413-454), in source order.
 // RG_PAIRPAR_RESIDENT (kernels.h): resident CTAs per SM the register budget is cut for (the
@@ -45,17 +45,16 @@ int set_error(int code, const std::string& msg);
 // S sinks x STRIDE threads per CTA, four pair terms per thread and tile (J = 4 STRIDE sources).
 // S sets the number of CTAs, ceil(sinks / S): the tuner picks the S whose grid fills the last
 // wave of resident CTAs best, since every CTA of a block runs the same sources and so takes the
-// same time.  Launched for the astrocentric frame.
-template <int S, int STRIDE, bool ASTRO>
+// same time.
+template <int S, int STRIDE>
 __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pairpar(GravArgs g)
 {
     constexpr int NT = S * STRIDE;
     constexpr int JPT = 4;           // terms per thread per tile
     constexpr int J = JPT * STRIDE;  // sources per tile
-    constexpr int JA = ASTRO ? J : 1;
     __shared__ double tx[J * S], ty[J * S], tz[J * S];
     __shared__ double sx[J], sy[J], sz[J], sm[J], sR[J], srho[J];
-    __shared__ double sind[3][JA];  // ASTRO: the sources' indirect terms
+    __shared__ double sind[3][J];  // the sources' indirect terms
     __shared__ int sid[J];
 
     const Tile tile = g.tiles[blockIdx.x];
@@ -76,7 +75,7 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
     const int bc = t / S;  // phase-B component (0, 1, 2) for t < 3 S
     const double* Tb = bc == 0 ? tx : (bc == 1 ? ty : tz);
     double acc = 0.0;
-    if (ASTRO && t < 3 * S && sink_ok) acc = g.astro[bc * g.astro_stride + i];
+    if (t < 3 * S && sink_ok) acc = g.astro[bc * g.astro_stride + i];
 
     for (int j0 = tile.src_begin; j0 < tile.src_end; j0 += J) {
         const int nj = min(J, tile.src_end - j0);
@@ -85,11 +84,9 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
             sx[q] = g.px[j]; sy[q] = g.py[j]; sz[q] = g.pz[j];
             sm[q] = g.mass[j]; sR[q] = g.radius[j]; sid[q] = g.id[j];
             srho[q] = g.hill ? g.rho[j] : 0.0;
-            if (ASTRO) {
-                sind[0][q] = g.astro[3 * g.astro_stride + j];
-                sind[1][q] = g.astro[4 * g.astro_stride + j];
-                sind[2][q] = g.astro[5 * g.astro_stride + j];
-            }
+            sind[0][q] = g.astro[3 * g.astro_stride + j];
+            sind[1][q] = g.astro[4 * g.astro_stride + j];
+            sind[2][q] = g.astro[5 * g.astro_stride + j];
         }
         __syncthreads();
 #pragma unroll
@@ -104,19 +101,13 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
             tz[q * S + s] = o.tz;
         }
         __syncthreads();
-        if (t < 3 * S) {
-            if (ASTRO) {
-                if (active) {
-                    const double* Ib = sind[bc < 3 ? bc : 0];
-                    for (int q = 0; q < nj; q++)
-                        if (j0 + q != i && 0 <= sid[q]) {
-                            acc = acc + Tb[q * S + s];
-                            acc = acc - Ib[q];
-                        }
+        if (t < 3 * S && active) {
+            const double* Ib = sind[bc < 3 ? bc : 0];
+            for (int q = 0; q < nj; q++)
+                if (j0 + q != i && 0 <= sid[q]) {
+                    acc = acc + Tb[q * S + s];
+                    acc = acc - Ib[q];
                 }
-            } else {
-                for (int q = 0; q < nj; q++) acc = acc + Tb[q * S + s];
-            }
         }
         __syncthreads();
     }
@@ -322,13 +313,11 @@ __global__ void astro_terms_kernel(const double* __restrict__ x, const double* _
 int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
-    if (g.astro) {
-        switch (S) {
-        case 8: grav_fp64_pairpar<8, 32, true><<<g.n_tiles, 256, 0, st>>>(g); break;
-        case 16: grav_fp64_pairpar<16, 16, true><<<g.n_tiles, 256, 0, st>>>(g); break;
-        case 32: grav_fp64_pairpar<32, 8, true><<<g.n_tiles, 256, 0, st>>>(g); break;
-        default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 16 or 32 in the astrocentric frame");
-        }
+    switch (S) {
+    case 8: grav_fp64_pairpar<8, 32><<<g.n_tiles, 256, 0, st>>>(g); break;
+    case 16: grav_fp64_pairpar<16, 16><<<g.n_tiles, 256, 0, st>>>(g); break;
+    case 32: grav_fp64_pairpar<32, 8><<<g.n_tiles, 256, 0, st>>>(g); break;
+    default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 16 or 32 in the astrocentric frame");
     }
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
