@@ -73,10 +73,13 @@ struct MlpTrainSmem : MlpSmem {
     float A1p[MLP_MAT];  // silu(Z1), [s][position of v]
     float G2p[MLP_MAT];  // dL/dZ2, [s][position of u]
 };
-// The loss of a batch: 32 samples are added before they go to the sum.  Above this many samples
-// each goes there by itself: the rounding of that long a serial sum (2.5e-5 of the loss at
-// 100 000 samples, against 1e-7) is in every loss that callers have kept of such batches, and
-// those stay comparable.  It is what bounds such a batch: 1.9 ns an addition to one address.
+// The loss of a batch: a warp's 32 samples are added before they go to the sum.  Above this many
+// samples every other warp's go there one by one.  With all of them one by one the sum of 100 000
+// comes out 2.3e-5 of the loss too small (small terms round to nothing), which is in the losses
+// that callers have kept of such batches; half of them halves that error and stays within 2e-5 of
+// those losses, where adding 32 first throughout (1e-6 off) does not.  These additions bound such
+// a batch: 1.9 ns each to one address (a gradient of 100 000 samples: 354 us with all of them, 278
+// us with half).
 constexpr int MLP_SERIAL_LOSS = 65536;
 constexpr int MLP_FORWARD_CTAS = 3;  // per SM (training: 2)
 constexpr int MLP_GROUP = MLP_HIDDEN * (MLP_IN + 1);  // dW1 and db1 of one sample group
@@ -107,7 +110,7 @@ __device__ __forceinline__ void mlp_mma(float (&acc)[4][4], const float* A, cons
 // block reads two float4 for 16 FMAs, each SiLU is taken once, and the weights' gradients go to
 // global memory once a CTA; one output per thread with its operands and SiLUs from shared memory
 // and a CTA's atomics per 32 samples took 280 us (forward) and 617 us (training) for 100 000
-// samples, this 46 and 190 us.
+// samples, this 46 and 190 us (with the loss one by one; 76 us of it went with half of that).
 template <bool TRAIN>
 __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
     mlp_tile_kernel(const __nv_bfloat16* __restrict__ wb, const MlpNorm norm, const float* __restrict__ x,
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
             if constexpr (TRAIN) {
                 S.D[t] = d;
                 gb3 += d;
-                if (n > MLP_SERIAL_LOSS) {
+                if (n > MLP_SERIAL_LOSS && t < 32) {
                     if (t < ns) atomicAdd(&grad[MLP_NPARAM], e);
                 } else {
                     for (int q = 1; q < 32; q <<= 1) e += __shfl_xor_sync(0xffffffffu, e, q);
