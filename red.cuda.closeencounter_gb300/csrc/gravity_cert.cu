@@ -306,7 +306,9 @@ struct CertPrepArgs {
     const int* sys_base;    // first body of each system, or nullptr: one system of n bodies
     const int* sys_n;       // and its bodies
     const int* sys_active;
+    int n_sys;
     int n;
+    int blocks;             // CTAs per system
     int screen;
     float* rows;
     long long stride;
@@ -328,17 +330,21 @@ __device__ __forceinline__ float magnitude(const double* v, long long k)
     return __uint_as_float((h - (896u << 20)) << 3) * 1.000002f;
 }
 
-// One CTA per PREP_NT bodies of a system; each CTA first takes the maxima over the whole system
+// One CTA per PREP_NT bodies of a system, the systems one after the other over the whole grid (an
+// ensemble has more of them than a grid has rows); each CTA first takes the maxima over its system
 // (a few reads per thread from L2: less than a second launch costs).  The grid must not be
 // coarsened by a few bodies far out (ejected ones), so its range ends at 16 times the mean
 // |coordinate|; bodies beyond it are marked (NaN) and taken exactly.
 __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 {
-    const int sys = blockIdx.y;
-    if (blockIdx.x == 0 && sys == 0 && threadIdx.x == 0) *a.n_list = 0u;
+    const long long cta = blockIdx.x + (long long)gridDim.x * blockIdx.y;
+    const long long sys_of = cta / a.blocks;
+    if (sys_of >= a.n_sys) return;
+    const int sys = (int)sys_of, block = (int)(cta - sys_of * a.blocks);
+    if (cta == 0 && threadIdx.x == 0) *a.n_list = 0u;
     const int b0 = a.sys_base ? a.sys_base[sys] : 0, b1 = b0 + (a.sys_base ? a.sys_n[sys] : a.n);
-    const int j = b0 + blockIdx.x * PREP_NT + threadIdx.x;
-    if (b0 + blockIdx.x * PREP_NT >= b1 || (a.sys_active && !a.sys_active[sys])) return;
+    const int j = b0 + block * PREP_NT + threadIdx.x;
+    if (b0 + block * PREP_NT >= b1 || (a.sys_active && !a.sys_active[sys])) return;
     __shared__ float red[PREP_NT / 32][8];
     __shared__ float all[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -403,7 +409,7 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
     }
     int flat_bits = 0;
     for (int q = 0; q < 3; q++) flat_bits |= __syncthreads_and(flat[q]) ? 1 << q : 0;
-    if (blockIdx.x == 0 && threadIdx.x < 6)
+    if (block == 0 && threadIdx.x < 6)
         a.scale[8 * sys + threadIdx.x] = threadIdx.x < 2 ? all[threadIdx.x]
                                                          : (threadIdx.x < 5 ? all[threadIdx.x + 3] : __int_as_float(flat_bits));
     if (j >= b1) return;
@@ -779,9 +785,12 @@ int launch_cert_prep(const GravArgs& g, const int* sys_base, const int* sys_n, i
                      cudaStream_t st)
 {
     if (max_n <= 0 || n_sys <= 0) return 0;
-    CertPrepArgs a{g.px, g.py, g.pz, g.mass, g.radius, g.hill ? g.rho : nullptr, g.id, sys_base, sys_n, g.sys_active, max_n,
-                   g.record || g.hill, cr.rows, cr.stride, cr.n_list, cr.scale};
-    cert_prep_kernel<<<dim3((max_n + PREP_NT - 1) / PREP_NT, n_sys), PREP_NT, 0, st>>>(a);
+    const int blocks = (max_n - 1) / PREP_NT + 1;
+    CertPrepArgs a{g.px, g.py, g.pz, g.mass, g.radius, g.hill ? g.rho : nullptr, g.id, sys_base, sys_n, g.sys_active, n_sys,
+                   max_n, blocks, g.record || g.hill, cr.rows, cr.stride, cr.n_list, cr.scale};
+    const long long ctas = (long long)blocks * n_sys, row = 1ll << 30;  // (a grid has 2^31 - 1 columns, 65 535 rows)
+    const dim3 grid((unsigned)(ctas < row ? ctas : row), (unsigned)((ctas + row - 1) / row));
+    cert_prep_kernel<<<grid, PREP_NT, 0, st>>>(a);
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;
 }
