@@ -368,7 +368,9 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
                 v[3] += z;
                 v[4] += 1.0f;
             }
-            if (a.screen && pass == 0 && k >= b0 + HEAD) {
+            // (a merged body waits at 1e20 AU with id < 0: one of them would open the Hill screen to every
+            // pair; a step of 8003 bodies 3.3 -> 14.8 ms)
+            if (a.screen && pass == 0 && k >= b0 + HEAD && 0 <= a.id[k]) {
                 v[5] = fmaxf(v[5], magnitude(a.radius, k));
                 v[6] = fmaxf(v[6], magnitude(a.mass, k));
                 if (a.rho) v[7] = fmaxf(v[7], magnitude(a.rho, k));
