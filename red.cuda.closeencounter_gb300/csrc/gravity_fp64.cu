@@ -221,10 +221,24 @@ struct RowSmem {
     std::conditional_t<LIST, NoRules, GroupRowSmem<640, RowShape<LIST, TERMS>::SUM_WARPS>> sum[3];
 };
 
-// LIST: the rows *n_list of `list` (part: components to add), without event tests
+// the event tests of body i with the sources from sink_end on (a pair's tests are its later body's), by
+// a CTA; kept out of the row kernel's own code, which the tests inlined slow by an eighth
+__device__ __noinline__ void row_events(const GravArgs& g, const Tile& tile, int i)
+{
+    if (!(0 < g.id[i])) return;
+    for (int j = tile.sink_end + (int)threadIdx.x; j < min(i, tile.src_end); j += blockDim.x) {
+        PairOut o;
+        if (0 <= g.id[j])
+            pair_term(g, tile, i, j, g.px[i], g.py[i], g.pz[i], g.radius[i], g.mass[i], g.hill ? g.rho[i] : 0.0, g.px[j],
+                      g.py[j], g.pz[j], g.mass[j], g.radius[j], g.hill ? g.rho[j] : 0.0, o);
+    }
+}
+
+// LIST: the rows *n_list of `list` (part: components to add; sink_end: the event tests of sources from
+// there on are the row's too)
 template <bool LIST, int TERMS>
 __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LIST, TERMS>::CTAS)
-    grav_fp64_rows(GravArgs g, const Tile* list, const unsigned int* n_list)
+    grav_fp64_rows(const __grid_constant__ GravArgs g, const Tile* list, const unsigned int* n_list)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
     using Shape = RowShape<LIST, TERMS>;
@@ -276,6 +290,7 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
             __syncthreads();
         }
         if (adds && (int)threadIdx.x == LANES * comp) (comp == 0 ? g.ax : comp == 1 ? g.ay : g.az)[i] = acc;
+        if (LIST && tile.sink_end < min(i, tile.src_end) && (g.record || g.hill)) row_events(g, tile, i);
     }
 }
 

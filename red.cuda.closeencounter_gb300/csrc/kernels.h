@@ -84,7 +84,8 @@ struct CertRows {
     float* rows;       // 8 FP32 rows of `stride` (cert_stride)
     long long stride;
     float* scale;      // 8 per system
-    Tile* list;        // rows left over: one sink each, part = its components (bits); one slot per body
+    Tile* list;        // rows left over: one sink each, part = its components (bits), sink_end = the first
+                       // source it is to test for events (src_end: none); one slot per body
     unsigned int* n_list;
 };
 long long cert_stride(int n, int n_sys);
