@@ -534,7 +534,12 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
         }
         if (g.hill) {
             const float inv3M = (float)(1.0 / (3.0 * g.mass[tile.base]));
-            const float lim = cbrtf(g.hill_f3_f * (mi + sc[3]) * inv3M) * 0.5f * (__double2float_ru(g.rho[i]) + sc[4]) * 1.001f;
+            const float k3 = cbrtf(g.hill_f3_f * (mi + sc[3]) * inv3M), rho = __double2float_ru(g.rho[i]);
+            float lim = k3 * 0.5f * (rho + sc[4]);
+            // (a source at the distance d is at most d further from the star: one body far out does not
+            // open the screens of the others)
+            if (k3 < 1.0f) lim = fminf(lim, k3 * rho / (1.0f - 0.5f * k3));
+            lim *= 1.001f;
             event_cut = fmaxf(event_cut, lim * lim);
         }
     }

@@ -35,6 +35,13 @@ def _hill_ms(d, factor):
     return best
 
 
+def test_distant_bodies_leave_the_hill_screen_narrow(gpulib):
+    """1000 AU out: the screen of every other body stays as wide as without them (with the
+    largest star distance in it, the step took twice as long)."""
+    whole, far = _hill_ms(_disk(4000, 0, 0.0), 0.0), _hill_ms(_disk(4000, 1, 1000.0), 0.0)
+    assert far < 1.35 * whole, (whole, far)
+
+
 @pytest.mark.parametrize("where", ["far", "high"])
 def test_bodies_outside_the_grid_do_not_last_longest(gpulib, where):
     """A body 100 AU out, or 1 AU above the disk, has every pair taken exactly: by the row kernel, not by
