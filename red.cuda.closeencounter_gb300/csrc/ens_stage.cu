@@ -25,7 +25,7 @@ int set_error(int code, const std::string& msg);
 
 namespace {
 
-constexpr int HMAX = 3;  // heavy bodies of a disk
+constexpr int HMAX = STAGE_SYM_HEAVY;  // heavy bodies of a disk
 
 // df_mul with its product's rounding kept out of multiply-adds, as the stage sums' unit is built
 __device__ __forceinline__ DF mul_nc(DF a, DF b)
@@ -358,6 +358,8 @@ __global__ void __launch_bounds__(256, DF_SYM_RESIDENT) ens_stage_sym(StageSymAr
 int launch_ens_stage_sym(const StageSymArgs& a, int nterm, int n_cta, cudaStream_t st)
 {
     if (n_cta <= 0) return 0;
+    // the term counts of the RKF7(8) stages (rk_tables.h); any other would leave the stage unwritten
+    if (nterm < 1 || nterm > 9 || nterm == 5) return set_error(RG_ERR_ARG, "a stage of so many terms has no kernel");
     cudaLaunchAttribute pdl[1];
     pdl[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     pdl[0].val.programmaticStreamSerializationAllowed = 1;
