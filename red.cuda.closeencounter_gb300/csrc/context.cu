@@ -144,7 +144,7 @@ struct rg_ctx {
         int row_base;   // few-sink groups: first row in the terms buffer
         int rows;       // few-sink groups: rows
         int max_src;    // few-sink groups: largest source count of a tile
-        int max_sinks;  // few-sink groups: widest tile
+        int max_sinks;  // widest tile
     };
     std::vector<Group> plan[2];
     bool swarm = false, swarm_fp64 = false;  // a disk for swarm_step.cu, swarm_fp64.cu
@@ -361,13 +361,14 @@ int set_param_dev(rg_ctx* c, int i)
 
 // --------------------------------------------------------------------- launch plan
 enum {
-    GROUP_PAIRPAR = 0,
+    GROUP_CERT = 0,       // certified terms, and the rows they leave over
     GROUP_ROWSEQ = 1,
     GROUP_FP64_ROWS = 2,
     GROUP_MIXED = 3,
     GROUP_DF_ROWSEQ = 4,  // mixed mode: the row kernel in double-float arithmetic
     GROUP_DF_FEW = 5,     // mixed mode: few heavy sinks in double-float arithmetic
     GROUP_DF_SYM = 6,     // mixed mode: heavy-light pairs once for both rows (grav_df_sym)
+    GROUP_PAIRPAR = 7,
 };
 // light bodies per symmetric tile of one disk, about: one per thread of a 256-thread CTA up to
 // a wave of resident CTAs, so that a disk of a thousand bodies spreads over several SMs (the
@@ -492,12 +493,18 @@ void build_tiles(rg_ctx* c)
             continue;
         }
         const int light0 = b.block == 0 ? std::max(b.s0, std::min(n_heavy, b.s1)) : b.s0;
-        // the heavy rows' sums are as small as their terms, so their integers do not save the FP64
-        // terms (gravity_cert.cu): exact serial row sums, beside the light rows
-        // (small blocks: every row -- FP64_ROW_PAIRS)
-        const int pair0 = (int64_t)ns * b.src1 <= FP64_ROW_PAIRS ? b.s1 : (light0 - b.s0 <= FEW_BLOCK_SINKS ? light0 : b.s0);
-        add_group(0, GROUP_FP64_ROWS, b.s0, pair0, b.src1, b.block, 1);
-        add_group(0, GROUP_PAIRPAR, pair0, b.s1, b.src1, b.block, c->pairpar_S);
+        const Fp64Form form = fp64_block_form(ns, (int64_t)ns * b.src1);
+        if (form == FP64_FORM_PAIRPAR) {
+            PairparSinks sinks;
+            sinks.add(ns, b.src1);
+            add_group(0, GROUP_PAIRPAR, b.s0, b.s1, b.src1, b.block, sinks.best(RG_PAIRPAR_RESIDENT, c->n_sm));
+        } else {
+            // the heavy rows' sums are as small as their terms, so their integers do not save the FP64
+            // terms (gravity_cert.cu): exact serial row sums, beside the light rows
+            const int cert0 = form == FP64_FORM_ROWS ? b.s1 : (light0 - b.s0 <= FEW_BLOCK_SINKS ? light0 : b.s0);
+            add_group(0, GROUP_FP64_ROWS, b.s0, cert0, b.src1, b.block, 1);
+            add_group(0, GROUP_CERT, cert0, b.s1, b.src1, b.block, c->pairpar_S);
+        }
         add_group(1, GROUP_DF_FEW, b.s0, light0, b.src1, b.block, FEW_SINKS_MAX);
         add_group(1, GROUP_MIXED, light0, b.s1, b.src1, b.block, MIXED_SINKS_PER_TILE);
     }
@@ -658,11 +665,18 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
     // FP64: the few-sink rows (star, giants: their terms, then a long serial sum per row, whose
     // dependent FP64 additions set the evaluation's latency) on the side stream, beside the other
     // groups; they write other rows and append events atomically (collect_events sorts them)
-    bool fork_few = false;
+    // (and wide, shallow blocks beside certified ones: 103 massive bodies, 3000 planetesimals and 3000
+    // test particles 249 us one after the other, 229 side by side)
+    bool fork_few = false, fork_wide = false;
     if (c->gravity_mode == RG_GRAVITY_FP64) {
-        bool few = false, other = false;
-        for (const auto& gr : c->plan[0]) (gr.kind == GROUP_FP64_ROWS ? few : other) = true;
-        fork_few = few && other;
+        bool few = false, other = false, wide = false, cert_plan = false;
+        for (const auto& gr : c->plan[0]) {
+            (gr.kind == GROUP_FP64_ROWS ? few : other) = true;
+            wide = wide || gr.kind == GROUP_PAIRPAR;
+            cert_plan = cert_plan || gr.kind == GROUP_CERT;
+        }
+        fork_wide = wide && cert_plan;
+        fork_few = (few && other) || fork_wide;
     }
     if (fork_few) {
         RG_CUDA_CHECK(cudaEventRecord(c->ev_fork, c->st));
@@ -675,11 +689,11 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
         g.n_tiles = gr.n;
         switch (gr.kind) {
         case GROUP_PAIRPAR:
-            if (c->frame == RG_FRAME_ASTRO) {
-                rc = launch_grav_fp64_pairpar(g, c->pairpar_S, c->st);
-                c->n_kernels++;
-                break;
-            }
+            rc = launch_grav_fp64_pairpar(g, c->frame == RG_FRAME_ASTRO ? c->pairpar_S : gr.max_sinks,
+                                          fork_wide ? c->st2 : c->st);
+            c->n_kernels++;
+            break;
+        case GROUP_CERT:
             if (!split_done) {
                 rc = launch_cert_prep(g, nullptr, nullptr, 1, c->n_total(), c->cert, c->st);
                 split_done = true;
@@ -784,7 +798,7 @@ int gravity(rg_ctx* c, const double* pos, const double* vel, double* acc, int st
         }
         if (rc) break;
     }
-    if (cert && !rc) {  // the rows the pair-parallel kernel left over
+    if (cert && !rc) {  // the rows the certified kernel left over
         rc = launch_grav_fp64_list(g, c->cert, c->st);
         c->n_kernels++;
     }

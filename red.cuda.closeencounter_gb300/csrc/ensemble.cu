@@ -805,6 +805,7 @@ struct rg_ens {
     // gravity launch shapes (rg_ens_autotune): row-kernel source limit, sinks per FP64
     // pair-parallel CTA, sources per few-sink CTA (0: automatic)
     int rowseq_max_src = 64, pairpar_S = 16, few_chunk = 0;
+    int pairpar_sinks = 8;  // of a pair-parallel CTA
     std::vector<int> base, ntot;
     std::vector<std::array<int, 7>> cnt;
     std::vector<rg_param_t> p;
@@ -963,14 +964,15 @@ constexpr long long ATTEMPT_CHUNK = 4096;  // attempts per graph launch at most
 // the FP64 plan uses the first three kinds; the mixed-precision plan uses MIXED, DF_ROWSEQ,
 // DF_FEW and DF_SYM (double-float heavy pairs)
 enum {
-    GROUP_PAIRPAR = 0,
+    GROUP_CERT = 0,
     GROUP_ROWSEQ = 1,
     GROUP_FP64_ROWS = 2,
     GROUP_MIXED = 3,
     GROUP_DF_ROWSEQ = 4,
     GROUP_DF_FEW = 5,
     GROUP_DF_SYM = 6,  // heavy-light pairs once for both rows, with its systems' heavy rows
-    GROUP_KINDS = 7
+    GROUP_PAIRPAR = 7,
+    GROUP_KINDS = 8
 };
 constexpr int ENS_SYM_CHUNK = 2048;  // light bodies per symmetric tile about, unless tuned
 
@@ -1104,12 +1106,49 @@ void build_gravity_plan(rg_ens* e)
         hv[1][GROUP_DF_SYM].assign(by[1][GROUP_DF_SYM].size(), 0);
         for (size_t k = 0; k < sym_systems.size(); k++) sym_parts[sym_systems[k].sys] = parts[k];
     }
-    int64_t block_pairs = 0;  // of the blocks with many sinks and many sources, all disks
-    for (int s = 0; s < e->n_sys; s++) {
-        const int64_t nsi = e->n_si(s), nm = e->n_massive(s), nt = e->ntot[s];
-        for (const auto& k : {std::make_pair(nsi, nm), std::make_pair(nm - nsi, nsi), std::make_pair(nt - nm, nm)})
-            if (k.second > e->rowseq_max_src && k.first > ENS_FEW_BLOCK) block_pairs += k.first * k.second;
+    // The FP64 form of the blocks with many sources, all disks' together: of each kind of block those with
+    // many sinks (without the wide and shallow ones all or none certified), and [3] the rows of few
+    // sinks: blocks of them, and the heavy rows beside certified ones (their terms are as large as their
+    // sums, gravity_cert.cu)
+    const auto block_of = [&](int s, int k, int64_t* sinks, int64_t* sources) {
+        const int64_t nsi = e->n_si(s), nm = e->n_massive(s);
+        *sinks = k == 0 ? nsi : (k == 1 ? nm - nsi : e->ntot[s] - nm);
+        *sources = k == 1 ? nsi : nm;
+        return *sinks > 0 && *sources > e->rowseq_max_src;
+    };
+    const auto heavy_of = [&](int s) { return std::min(e->n_si(s), e->cnt[s][0] + e->cnt[s][1] + e->cnt[s][2]); };
+    int64_t rows[4] = {0, 0, 0, 0}, pairs[4] = {0, 0, 0, 0}, ns, nsrc;
+    for (int s = 0; s < e->n_sys; s++)
+        for (int k = 0; k < 3; k++)
+            if (block_of(s, k, &ns, &nsrc)) {
+                const int q = ns > ENS_FEW_BLOCK ? k : 3;
+                rows[q] += ns;
+                pairs[q] += ns * nsrc;
+            }
+    Fp64Form form[4];
+    bool cert = false;
+    int64_t rest = 0;
+    for (int k = 0; k < 3; k++) {
+        form[k] = fp64_block_form(rows[k], pairs[k]);
+        if (form[k] != FP64_FORM_PAIRPAR) rest += pairs[k];
+        cert = cert || form[k] == FP64_FORM_CERT;
     }
+    for (int k = 0; k < 3; k++)
+        if (form[k] == FP64_FORM_ROWS && (cert || rest > FP64_ROW_PAIRS)) form[k] = FP64_FORM_CERT;
+    for (int s = 0; s < e->n_sys; s++)
+        if (block_of(s, 0, &ns, &nsrc) && ns > ENS_FEW_BLOCK && form[0] == FP64_FORM_CERT && heavy_of(s) <= ENS_FEW_BLOCK) {
+            rows[3] += heavy_of(s);
+            pairs[3] += heavy_of(s) * nsrc;
+        }
+    form[3] = fp64_wide(rows[3], pairs[3]) ? FP64_FORM_PAIRPAR : FP64_FORM_ROWS;
+    // where the pair-parallel kernel runs, short rows are a few CTAs more of it (4 disks of 103 bodies
+    // and 2000 test particles: 1105 us an attempt with a launch for the rows, 991 without)
+    if (std::find(form, form + 4, FP64_FORM_PAIRPAR) != form + 4)
+        for (int k = 0; k < 4; k++)
+            if (form[k] == FP64_FORM_ROWS && pairs[k] <= 256 * rows[k]) form[k] = FP64_FORM_PAIRPAR;
+    const int few_kind = form[3] == FP64_FORM_PAIRPAR ? GROUP_PAIRPAR : GROUP_FP64_ROWS;
+    std::vector<Tile> wide;  // the pair-parallel kernel's blocks, to be cut when all are known
+    PairparSinks sinks;
     for (int s = 0; s < e->n_sys; s++) {
         const int b = e->base[s];
         const int nsi = e->n_si(s), nm = e->n_massive(s), nt = e->ntot[s];
@@ -1120,6 +1159,11 @@ void build_gravity_plan(rg_ens* e)
             int s0, s1, src1, block;
         } blks[3] = {{0, nsi, nm, 0}, {nsi, nm, nsi, 1}, {nm, nt, nm, 2}};
         auto add = [&](int mode, int kind, int s0, int s1, int src1, int block, int step) {
+            if (kind == GROUP_PAIRPAR && s0 < s1) {
+                wide.push_back(Tile{b + s0, b + s1, b, b + src1, s, b, block, 0});
+                sinks.add(s1 - s0, src1);
+                return;
+            }
             for (int q = s0; q < s1; q += step) {
                 by[mode][kind].push_back(Tile{b + q, b + std::min(q + step, s1), b, b + src1, s, b, block, 0});
                 hv[mode][kind].push_back(b + std::min(n_heavy, src1));
@@ -1132,20 +1176,32 @@ void build_gravity_plan(rg_ens* e)
                 if (!(sym[s] && k.block == 1))  // a symmetric system's light rows: the segments above
                     add(1, GROUP_DF_ROWSEQ, k.s0, k.s1, k.src1, k.block, 128);
             } else if (k.s1 - k.s0 <= ENS_FEW_BLOCK) {
-                add(0, GROUP_FP64_ROWS, k.s0, k.s1, k.src1, k.block, 1);
+                add(0, few_kind, k.s0, k.s1, k.src1, k.block, 1);
                 if (!(sym[s] && k.block == 0))  // a symmetric system's heavy rows come with its tiles
                     add(1, GROUP_DF_FEW, k.s0, k.s1, k.src1, k.block, FEW_SINKS_MAX);
             } else {
                 const int light0 = k.block == 0 ? std::max(k.s0, std::min(n_heavy, k.s1)) : k.s0;
-                // heavy rows: exact serial sums (their terms are as large as the sums, gravity_cert.cu)
-                const int pair0 = block_pairs <= FP64_ROW_PAIRS ? k.s1 : (light0 - k.s0 <= ENS_FEW_BLOCK ? light0 : k.s0);
-                add(0, GROUP_FP64_ROWS, k.s0, pair0, k.src1, k.block, 1);
-                add(0, GROUP_PAIRPAR, pair0, k.s1, k.src1, k.block, e->pairpar_S);  // S sinks per tile
+                if (form[k.block] != FP64_FORM_CERT) {
+                    add(0, form[k.block] == FP64_FORM_PAIRPAR ? GROUP_PAIRPAR : GROUP_FP64_ROWS, k.s0, k.s1, k.src1, k.block, 1);
+                } else {
+                    const int cert0 = light0 - k.s0 <= ENS_FEW_BLOCK ? light0 : k.s0;
+                    add(0, few_kind, k.s0, cert0, k.src1, k.block, 1);
+                    add(0, GROUP_CERT, cert0, k.s1, k.src1, k.block, e->pairpar_S);  // S sinks per tile
+                }
                 add(1, GROUP_DF_FEW, k.s0, light0, k.src1, k.block, FEW_SINKS_MAX);
                 add(1, GROUP_MIXED, light0, k.s1, k.src1, k.block, MIXED_SINKS_PER_TILE);
             }
         }
     }
+    e->pairpar_sinks = sinks.best(RG_PAIRPAR_RESIDENT, e->n_sm);
+    for (const Tile& w : wide)
+        for (int q = w.sink_begin; q < w.sink_end; q += e->pairpar_sinks) {
+            Tile t = w;
+            t.sink_begin = q;
+            t.sink_end = std::min(q + e->pairpar_sinks, w.sink_end);
+            by[0][GROUP_PAIRPAR].push_back(t);
+            hv[0][GROUP_PAIRPAR].push_back(0);
+        }
     for (int mode = 0; mode < 2; mode++) {
         e->plan[mode].clear();
         for (int kind = 0; kind < GROUP_KINDS; kind++) {
@@ -1356,7 +1412,8 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
         g.tiles = e->d_tiles + gr.off;
         g.n_tiles = gr.n;
         switch (gr.kind) {
-        case GROUP_PAIRPAR:
+        case GROUP_PAIRPAR: rc = launch_grav_fp64_pairpar(g, e->pairpar_sinks, e->st); e->n_kernels++; break;
+        case GROUP_CERT:
             if (!split_done) {
                 rc = launch_cert_prep(g, e->d_base, e->d_ntot, e->n_sys, e->max_n, e->cert, e->st);
                 split_done = true;
@@ -1418,7 +1475,7 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
         }
         if (rc) break;
     }
-    if (cert && !rc) {  // the rows the pair-parallel kernel left over
+    if (cert && !rc) {  // the rows the certified kernel left over
         rc = launch_grav_fp64_list(g, e->cert, e->st);
         e->n_kernels++;
     }
@@ -1822,15 +1879,15 @@ int create_impl(int n_sys, const rg_counts_t* counts, const rg_vec_t* r, const r
     chk(dalloc(&e->d_type, nt));
     chk(dalloc(&e->d_base_of, nt));
     chk(dalloc((char**)&e->d_split, SPLIT_POS_BYTES * nt));
-    bool pairpar = false;  // a disk with a block for the pair-parallel kernel
+    bool certified = false;  // a disk with a block that may go to the certified kernel
     for (int s = 0; s < n_sys; s++) {
         e->max_n = std::max(e->max_n, e->ntot[s]);
-        pairpar = pairpar || e->n_si(s) > ENS_FEW_BLOCK || e->ntot[s] - e->n_massive(s) > ENS_FEW_BLOCK;
+        certified = certified || e->n_si(s) > ENS_FEW_BLOCK || e->ntot[s] - e->n_massive(s) > ENS_FEW_BLOCK;
     }
     e->cert.stride = cert_stride((int)nt, n_sys);
-    chk(dalloc(&e->cert.rows, pairpar ? (size_t)(8 * e->cert.stride) : 1));
+    chk(dalloc(&e->cert.rows, certified ? (size_t)(8 * e->cert.stride) : 1));
     chk(dalloc(&e->cert.scale, 8 * ns));
-    chk(dalloc(&e->cert.list, pairpar ? nt : 1));
+    chk(dalloc(&e->cert.list, certified ? nt : 1));
     chk(dalloc(&e->cert.n_list, 1));
     chk(dalloc(&e->d_rf, nt));
     chk(dalloc(&e->d_mass_f2, nt));

@@ -16,8 +16,8 @@
 // segments, row_sum.h) for rows of many sources in blocks of few pairs, and for the rows that
 // gravity_cert.cu, which takes the large blocks, leaves over; the row-serial kernel (thread per
 // sink) for blocks with few sources per sink (planetesimals x 3 massive bodies); and the
-// pair-parallel kernel (S x J terms into shared memory, 3 S threads add them) for the
-// astrocentric frame.
+// pair-parallel kernel (S x J terms into shared memory, 3 S threads add them) for blocks of many
+// sinks with a hundred sources or so, and the astrocentric frame.
 #include <atomic>
 #include <string>
 #include <type_traits>
@@ -34,8 +34,9 @@ namespace redgb {
 int set_error(int code, const std::string& msg);
 
 // ---------------------------------------------------------------------------------------
-// Pair-parallel kernel: CTA = S sinks, source tiles of J = 1024 / S, for the astrocentric frame
-// of the reference's CPU path -- each sink starts from the star's pull
+// Pair-parallel kernel: CTA = S sinks, source tiles of J = 1024 / S, for blocks of many sinks with a
+// hundred sources or so (fp64_block_form, plan_tools.h) and the astrocentric frame (ASTRO) of the
+// reference's CPU path -- there each sink starts from the star's pull
 // and, for every source it interacts with, adds the direct term and then subtracts the
 // source's indirect term (pp_disk.cu:413-454), in source order.
 // RG_PAIRPAR_RESIDENT (kernels.h): resident CTAs per SM the register budget is cut for (the
@@ -45,8 +46,10 @@ int set_error(int code, const std::string& msg);
 // S sinks x STRIDE threads per CTA, four pair terms per thread and tile (J = 4 STRIDE sources).
 // S sets the number of CTAs, ceil(sinks / S): the tuner picks the S whose grid fills the last
 // wave of resident CTAs best, since every CTA of a block runs the same sources and so takes the
-// same time.
-template <int S, int STRIDE>
+// same time.  In the barycentric frame the plan takes the S of the least waves x steps (PairparSinks):
+// 5000 / 20 000 sinks of 65 sources 14 / 49 us, a CTA per row 77 / 287 us, certified 41 / 70 us;
+// an RKF7(8) attempt of 64 / 256 disks of 103 / 73 bodies 529 / 963 us, in rows 1625 / 4095 us.
+template <int S, int STRIDE, bool ASTRO>
 __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pairpar(GravArgs g)
 {
     constexpr int NT = S * STRIDE;
@@ -54,7 +57,7 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
     constexpr int J = JPT * STRIDE;  // sources per tile
     __shared__ double tx[J * S], ty[J * S], tz[J * S];
     __shared__ double sx[J], sy[J], sz[J], sm[J], sR[J], srho[J];
-    __shared__ double sind[3][J];  // the sources' indirect terms
+    __shared__ double sind[3][ASTRO ? J : 1];  // the sources' indirect terms
     __shared__ int sid[J];
 
     const Tile tile = g.tiles[blockIdx.x];
@@ -75,7 +78,7 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
     const int bc = t / S;  // phase-B component (0, 1, 2) for t < 3 S
     const double* Tb = bc == 0 ? tx : (bc == 1 ? ty : tz);
     double acc = 0.0;
-    if (t < 3 * S && sink_ok) acc = g.astro[bc * g.astro_stride + i];
+    if (ASTRO && t < 3 * S && sink_ok) acc = g.astro[bc * g.astro_stride + i];
 
     for (int j0 = tile.src_begin; j0 < tile.src_end; j0 += J) {
         const int nj = min(J, tile.src_end - j0);
@@ -84,9 +87,11 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
             sx[q] = g.px[j]; sy[q] = g.py[j]; sz[q] = g.pz[j];
             sm[q] = g.mass[j]; sR[q] = g.radius[j]; sid[q] = g.id[j];
             srho[q] = g.hill ? g.rho[j] : 0.0;
-            sind[0][q] = g.astro[3 * g.astro_stride + j];
-            sind[1][q] = g.astro[4 * g.astro_stride + j];
-            sind[2][q] = g.astro[5 * g.astro_stride + j];
+            if (ASTRO) {
+                sind[0][q] = g.astro[3 * g.astro_stride + j];
+                sind[1][q] = g.astro[4 * g.astro_stride + j];
+                sind[2][q] = g.astro[5 * g.astro_stride + j];
+            }
         }
         __syncthreads();
 #pragma unroll
@@ -101,13 +106,17 @@ __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pai
             tz[q * S + s] = o.tz;
         }
         __syncthreads();
-        if (t < 3 * S && active) {
-            const double* Ib = sind[bc < 3 ? bc : 0];
-            for (int q = 0; q < nj; q++)
-                if (j0 + q != i && 0 <= sid[q]) {
-                    acc = acc + Tb[q * S + s];
-                    acc = acc - Ib[q];
-                }
+        if (ASTRO) {
+            if (t < 3 * S && active) {
+                const double* Ib = sind[bc < 3 ? bc : 0];
+                for (int q = 0; q < nj; q++)
+                    if (j0 + q != i && 0 <= sid[q]) {
+                        acc = acc + Tb[q * S + s];
+                        acc = acc - Ib[q];
+                    }
+            }
+        } else if (t < 3 * S) {
+            for (int q = 0; q < nj; q++) acc = acc + Tb[q * S + s];
         }
         __syncthreads();
     }
@@ -328,11 +337,16 @@ __global__ void astro_terms_kernel(const double* __restrict__ x, const double* _
 int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st)
 {
     if (g.n_tiles <= 0) return 0;
+    auto launch = [&](auto kernel) { kernel<<<g.n_tiles, 256, 0, st>>>(g); };
     switch (S) {
-    case 8: grav_fp64_pairpar<8, 32><<<g.n_tiles, 256, 0, st>>>(g); break;
-    case 16: grav_fp64_pairpar<16, 16><<<g.n_tiles, 256, 0, st>>>(g); break;
-    case 32: grav_fp64_pairpar<32, 8><<<g.n_tiles, 256, 0, st>>>(g); break;
-    default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 16 or 32 in the astrocentric frame");
+    case 4:
+        if (g.astro) return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 8, 16 or 32 in the astrocentric frame");
+        launch(grav_fp64_pairpar<4, 64, false>);
+        break;
+    case 8: launch(g.astro ? grav_fp64_pairpar<8, 32, true> : grav_fp64_pairpar<8, 32, false>); break;
+    case 16: launch(g.astro ? grav_fp64_pairpar<16, 16, true> : grav_fp64_pairpar<16, 16, false>); break;
+    case 32: launch(g.astro ? grav_fp64_pairpar<32, 8, true> : grav_fp64_pairpar<32, 8, false>); break;
+    default: return set_error(RG_ERR_ARG, "pair-parallel sinks per CTA: 4, 8, 16 or 32");
     }
     RG_CUDA_CHECK(cudaGetLastError());
     return 0;

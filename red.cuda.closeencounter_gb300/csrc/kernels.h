@@ -73,10 +73,10 @@ struct EnergyArgs {
 
 int launch_energy(const EnergyArgs& a, cudaStream_t st);
 
-// resident pair-parallel CTAs per SM (the kernels are built for it: 80 registers, 256 threads)
+// resident pair-parallel CTAs per SM (the kernels are built for it: at most 80 registers, 256 threads)
 constexpr int RG_PAIRPAR_RESIDENT = 3;
-int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st);  // astrocentric frame
-// barycentric frame (gravity_cert.cu): launch_cert_prep writes an evaluation's rows and scales
+int launch_grav_fp64_pairpar(const GravArgs& g, int S, cudaStream_t st);  // S: sinks of a tile and CTA
+// certified terms (gravity_cert.cu), barycentric frame: launch_cert_prep writes an evaluation's rows and scales
 // (sys_base, sys_n: each system's first body and body count, or nullptr: one system of max_n
 // bodies), launch_grav_fp64_cert the tiles' sums (S: sinks per tile)
 // except those it lists, which launch_grav_fp64_list (gravity_fp64.cu) then adds
@@ -99,12 +99,6 @@ int launch_grav_fp64_rowseq(const GravArgs& g, cudaStream_t st);
 constexpr int FEW_SINKS_MAX = 8;  // sinks per few-sink tile (mixed mode)
 // FP64 rows of tiles of one sink each: exact terms added in order (gravity_fp64.cu)
 int launch_grav_fp64_rows(const GravArgs& g, int max_src, cudaStream_t st);  // max_src: a row's most sources
-// blocks of up to this many (sink, source) pairs go row by row, larger ones to gravity_cert.cu: a
-// row's latency is a few microseconds and its pairs cost five times as much.  Self-interacting
-// blocks of 400 / 1000 / 1300 / 1480 bodies on GB300: rows 18 / 55 / 85 / 101 us, gravity_cert.cu
-// 48 / 88 / 99 / 109 us; of 1700 and 2000, before the rows' last gain of a tenth, rows 146 / 195
-// us, gravity_cert.cu 124 / 149 us.
-constexpr int64_t FP64_ROW_PAIRS = 2250000;
 // mixed precision (gravity_mixed.cu): positions split into FP32 (hi, lo) once per evaluation
 struct SplitPos;
 constexpr int MIXED_SINKS_PER_TILE = 128;

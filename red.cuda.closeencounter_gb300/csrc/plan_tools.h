@@ -3,10 +3,68 @@
 #pragma once
 
 #include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <vector>
 
 namespace redgb {
+
+// The FP64 kernel of a block with more sources than the row-serial kernel takes (64): `rows` sinks and
+// `pairs` (sink, source) pairs, over all systems of an ensemble.
+//   rows (grav_fp64_rows): a CTA per row, 304 resident, 4.4 us a wave up to some 200 sources
+//   pair-parallel (grav_fp64_pairpar): S sinks a CTA; 30 to 45 ps a pair
+//   certified (grav_fp64_cert): 25 us more, then 2.7 ns a row of up to a few hundred sources
+// Square blocks go by their pairs: self-interacting blocks of 400 / 1000 / 1300 / 1480 bodies on
+// GB300: rows 18 / 55 / 85 / 101 us, certified 48 / 88 / 99 / 109 us; of 1700 and 2000, before the
+// rows' last gain of a tenth, rows 146 / 195 us, certified 124 / 149 us.  Wide, shallow ones by their
+// rows: blocks of 65 / 103 / 203 / 403 sources cost the same in rows and pair by pair at some 600 /
+// 700 / 1000 / 1600 sinks (5000 sinks of 65: 77 us in rows, 14 pair by pair, 41 certified), and are
+// certified from some 100 000 / 16 000 / 5000 / 2000 sinks on (20 000 of 203: 165 us pair by pair,
+// 105 certified).
+enum Fp64Form { FP64_FORM_ROWS, FP64_FORM_PAIRPAR, FP64_FORM_CERT };
+constexpr int64_t FP64_ROW_PAIRS = 2250000;
+inline bool fp64_wide(int64_t rows, int64_t pairs)  // rows > 400 + 2.8 sources
+{
+    return 5 * (rows - 400) * rows > 14 * pairs;
+}
+inline Fp64Form fp64_block_form(int64_t rows, int64_t pairs)
+{
+    if (!fp64_wide(rows, pairs)) return pairs <= FP64_ROW_PAIRS ? FP64_FORM_ROWS : FP64_FORM_CERT;
+    return pairs - 60 * rows <= 700000 ? FP64_FORM_PAIRPAR : FP64_FORM_CERT;  // rows (sources - 60)
+}
+
+// The sinks S of a pair-parallel CTA for the blocks added: 256 threads take four terms each of S x
+// 1024 / S pairs at a time, `resident` CTAs on each of n_sm SMs.  The S of the least waves x steps (a
+// CTA starts and sums for as long as two steps of terms take; half a wave's rounding counts: of 203
+// sources, 2000 sinks take 28 us with 8 and 44 with 16, 5000 take 72 and 63; 64 disks of 103 bodies
+// 565 us an attempt with 8, 529 with 16, 661 with 32).
+struct PairparSinks {
+    static constexpr int S[4] = {4, 8, 16, 32};
+    double ctas[4] = {}, steps[4] = {};
+    void add(int sinks, int sources)
+    {
+        for (int k = 0; k < 4; k++) {
+            const int stride = 256 / S[k], tile = 4 * stride, n = (sinks + S[k] - 1) / S[k];
+            ctas[k] += n;
+            steps[k] += (double)n * (sources / tile * 4 + (sources % tile + stride - 1) / stride + 2);
+        }
+    }
+    int best(int resident, int n_sm) const
+    {
+        int s = 8;
+        double least = -1.0;
+        for (int k = 0; k < 4; k++) {
+            if (ctas[k] <= 0.0) continue;
+            const double waves = ctas[k] / ((double)resident * std::max(n_sm, 1));
+            const double cost = (std::ceil(waves) + std::max(1.0, waves)) * steps[k] / ctas[k];
+            if (least < 0.0 || cost < least) {
+                least = cost;
+                s = S[k];
+            }
+        }
+        return s;
+    }
+};
 
 // Source chunks (grid.y) of the mixed tile kernel, two CTAs to an SM, for `sink_tiles` tiles of
 // sinks and `src_tiles` tiles of sources: as many as fit in one wave of CTAs, or, where that
