@@ -30,15 +30,17 @@
 // Error bound.  Coordinates are x = hi + lo + err with hi a multiple of a system-wide grid g (so
 // hi differences are exact) and lo in FP32; alpha = g 2^-24.  |lo| reaches 0.75 g (a coordinate
 // half-way between two grid points, and the split's own remainder): its rounding is 0.625 alpha at
-// most, the difference of two, up to 1.5 g, rounds by one alpha, so a displacement is good to
-// 2.25 alpha (DISP_ERR).  r^2 is summed with two-sums and the products' FMA errors, 1/r from rsqrt.approx (2^-22.9)
+// most, the difference of two, up to 1.5 g, rounds by one alpha.  Not all three at once: a rounding
+// of 0.5 alpha or more is a tie, which leaves lo an even multiple of alpha, and the difference of two
+// such ones is exact; so a displacement is good to (0.625 + 0.5 + 1) alpha (DISP_ERR; reached).
+// r^2 is summed with two-sums and the products' FMA errors, 1/r from rsqrt.approx (2^-22.9)
 // with its residual h = 1 - r^2 y0^2 formed by FMAs (3 2^-46), y^3 = y0^3 (1 + 1.5 h + 1.875 h^2);
 // every product keeps its FMA error term.  Relative error of w = m y^3: in units of 2^-44, 1.1
 // (h) + 0.6 (corr) + 1.0 (the error terms' and the term's last roundings) + 0.5 (their product
 // with the displacement's low part) + 0.5 (r^2's error terms) + 0.8 (the fast two-sum of the
 // remainder where its operands are in the other order) < 4.8, taken as 1.2 2^-42 with the
-// reference's own FP64 roundings (2^-49); plus 3 sqrt(3) 2.25 alpha / r = 11.7 alpha / r, taken as
-// 12.  A component's error is then at most w (|dx| (1.2 2^-42 + 12 alpha / r) + 3 alpha_c); |dx| is
+// reference's own FP64 roundings (2^-49); plus 3 sqrt(3) 2.125 alpha / r = 11.05 alpha / r, taken as
+// 11.2.  A component's error is then at most w (|dx| (1.2 2^-42 + 11.2 alpha / r) + 3 alpha_c); |dx| is
 // bounded by dx^2 / (2 eta) + eta / 2, which needs no absolute value in the packed form.
 #include <atomic>
 #include <string>
@@ -66,8 +68,8 @@ constexpr float BIG = 4.1e6f;         // |t / Q| / 2^16 below this (MAGIC's rang
 // accepted when f^2 + E < 1/4 - 2^-13: then |f| + E + 2^-13 < 1/2 (the rounding of f itself: 2^-23)
 constexpr float CERTAIN = 0.24987f;
 constexpr int64_t UNCERTAIN = 1ll << 36;  // terms this large are rarely certain (E > 2^-5)
-constexpr float DISP_ERR = 2.25f;     // of a displacement's component, in alpha
-constexpr float DISP_W = 12.0f;       // of w, in alpha / r
+constexpr float DISP_ERR = 2.125f;    // of a displacement's component, in alpha
+constexpr float DISP_W = 11.2f;       // of w, in alpha / r
 static_assert(DISP_W > 1.01f * 5.19616f * DISP_ERR, "3 sqrt(3) times a component's");
 constexpr float MIN_R2 = 8.3e-25f;    // 2^-80: closer pairs (and the sink itself) are taken exactly
 constexpr float MIN_MASS = 5.3e-23f;  // 2^-74: lighter masses have no exact split
@@ -131,7 +133,7 @@ __device__ __forceinline__ void regrid(float h, float l, float c, float& hi, flo
 // constants of the pair loop, each twice (packed)
 struct CertConst {
     f2 neg, one, two, c15, c1875, M, R;  // -1, 1, 2, 1.5, 1.875, MAGIC, RADIX
-    f2 Yk, Ya;                           // 2^16 1.2 2^-42, 2^16 12 alpha (the larger one)
+    f2 Yk, Ya;                           // 2^16 1.2 2^-42, 2^16 11.2 alpha (the larger one)
     f2 i2_xy, h_xy, a_xy;                // 1 / (2 eta), eta / 2, 2^16 3 alpha
     f2 i2_z, h_z, a_z;
 };
