@@ -230,10 +230,12 @@ struct RowSmem {
     std::conditional_t<LIST, NoRules, GroupRowSmem<640, RowShape<LIST, TERMS>::SUM_WARPS>> sum[3];
 };
 
-// the event tests of body i with the sources from sink_end on (a pair's tests are its later body's), by
-// a CTA; kept out of the row kernel's own code, which the tests inlined slow by an eighth
-__device__ __noinline__ void row_events(const GravArgs& g, const Tile& tile, int i)
+// the event tests of a listed row's body with the sources from sink_end on (a pair's tests are its later
+// body's), by a CTA; out of the row kernel's own code
+__device__ __noinline__ void row_events(const GravArgs& g, const Tile* row)
 {
+    const Tile tile = *row;
+    const int i = tile.sink_begin;
     if (!(0 < g.id[i])) return;
     for (int j = tile.sink_end + (int)threadIdx.x; j < min(i, tile.src_end); j += blockDim.x) {
         PairOut o;
@@ -299,7 +301,7 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
             __syncthreads();
         }
         if (adds && (int)threadIdx.x == LANES * comp) (comp == 0 ? g.ax : comp == 1 ? g.ay : g.az)[i] = acc;
-        if (LIST && tile.sink_end < min(i, tile.src_end) && (g.record || g.hill)) row_events(g, tile, i);
+        if (LIST && tile.sink_end < min(i, tile.src_end) && (g.record || g.hill)) row_events(g, list + row);
     }
 }
 
