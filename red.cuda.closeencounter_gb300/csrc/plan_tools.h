@@ -5,6 +5,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <utility>
 #include <vector>
 
 namespace redgb {
@@ -66,6 +67,32 @@ struct PairparSinks {
     }
 };
 
+// How long `sink_tiles` tiles of sinks take in source chunks of `tiles` of `src_tiles` source tiles each,
+// in source tiles: the CTAs, all whole chunks and then the last, shorter ones, go one after the
+// other to the slot that is free first, and a CTA starts for as long as a third of a source tile takes.
+constexpr double MIXED_START_COST = 0.3;
+inline double mixed_chunk_time(int sink_tiles, int src_tiles, int tiles, int slots)
+{
+    const int chunks = (src_tiles + tiles - 1) / tiles;
+    const int64_t whole = (int64_t)sink_tiles * (chunks - 1);
+    const double d = tiles + MIXED_START_COST, last = src_tiles - (chunks - 1) * tiles + MIXED_START_COST;
+    const int64_t waves = whole / slots, over = whole % slots;
+    // [time, slots free from then on], earliest first
+    std::vector<std::pair<double, int64_t>> free = {{waves * d, slots - over}};
+    if (over) free.push_back({(waves + 1) * d, over});
+    double end = (waves + (over ? 1 : 0)) * d;
+    int64_t left = sink_tiles;
+    for (size_t k = 0; left > 0; k++) {
+        const std::pair<double, int64_t> f = free[k];
+        const int64_t n = std::min(left, f.second);
+        left -= n;
+        end = std::max(end, f.first + last);
+        const std::pair<double, int64_t> next{f.first + last, n};
+        free.insert(std::upper_bound(free.begin() + (ptrdiff_t)k + 1, free.end(), next), next);
+    }
+    return end;
+}
+
 // Source chunks (grid.y) of the mixed tile kernel, two CTAs to an SM, for `sink_tiles` tiles of
 // sinks and `src_tiles` tiles of sources: as many as fit in one wave of CTAs, or, where that
 // leaves fewer, enough for 16 waves in chunks of at least six source tiles (a CTA starts with its
@@ -73,12 +100,31 @@ struct PairparSinks {
 // waves leaves the chip to the last of them).  Evaluations on GB300, one chunk per about 4 CTAs
 // an SM -> this rule: 1001 bodies 43.7 -> 28 us, 3001 60.5 -> 36 us, 16 385 358 -> 319 us,
 // 131 074 16.56 -> 15.7 ms.
+// Where the six tiles leave one to three waves, the count of the least mixed_chunk_time (the fewest on
+// a tie) is taken if it is better by 15 %, which is about how far that time is to be trusted (no CTA
+// runs alone on its SM in it, which is half as fast again): 6600 / 8500 / 9600 / 12 500 bodies
+// 87 / 128 / 138 / 208 us with six tiles, 77 / 110 / 128 / 200 us so; 13 000 and 14 000 bodies would
+// gain 14 and 5 % by it and lose 6.
 inline int mixed_chunk_count(int sink_tiles, int src_tiles, int n_sm)
 {
     const int64_t slots = 2 * (int64_t)std::max(n_sm, 1), tiles = std::max(sink_tiles, 1);
     const int64_t one_wave = slots / tiles;
     const int64_t many = std::min<int64_t>((16 * slots + tiles - 1) / tiles, src_tiles / 6);
-    return (int)std::max<int64_t>(1, std::min<int64_t>(std::max(one_wave, many), src_tiles));
+    int best = (int)std::max<int64_t>(1, std::min<int64_t>(std::max(one_wave, many), src_tiles));
+    if (src_tiles < 2) return best;
+    const auto time_of = [&](int n) {
+        return mixed_chunk_time((int)tiles, src_tiles, (src_tiles + n - 1) / n, (int)slots);
+    };
+    double least = time_of(best) / 1.15;
+    for (int n = 1; n <= src_tiles; n++) {
+        if (n > 1 && (src_tiles + n - 1) / n == (src_tiles + n - 2) / (n - 1)) continue;  // as with one chunk fewer
+        const double t = time_of(n);
+        if (t < least - 1e-9) {
+            least = t;
+            best = n;
+        }
+    }
+    return best;
 }
 
 // Segments of the symmetric heavy-light kernel (grav_df_sym).  `systems` holds one tile per
