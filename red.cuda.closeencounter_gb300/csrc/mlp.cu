@@ -73,14 +73,6 @@ struct MlpTrainSmem : MlpSmem {
     float A1p[MLP_MAT];  // silu(Z1), [s][position of v]
     float G2p[MLP_MAT];  // dL/dZ2, [s][position of u]
 };
-// The loss of a batch: a warp's 32 samples are added before they go to the sum.  Above this many
-// samples every other warp's go there one by one.  With all of them one by one the sum of 100 000
-// comes out 2.3e-5 of the loss too small (small terms round to nothing), which is in the losses
-// that callers have kept of such batches; half of them halves that error and stays within 2e-5 of
-// those losses, where adding 32 first throughout (1e-6 off) does not.  These additions bound such
-// a batch: 1.9 ns each to one address (a gradient of 100 000 samples: 354 us with all of them, 278
-// us with half).
-constexpr int MLP_SERIAL_LOSS = 65536;
 constexpr int MLP_FORWARD_CTAS = 3;  // per SM (training: 2)
 constexpr int MLP_GROUP = MLP_HIDDEN * (MLP_IN + 1);  // dW1 and db1 of one sample group
 static_assert(16 * MLP_GROUP <= 3 * MLP_MAT, "the groups' sums fit over the last three matrices");
@@ -110,7 +102,9 @@ __device__ __forceinline__ void mlp_mma(float (&acc)[4][4], const float* A, cons
 // block reads two float4 for 16 FMAs, each SiLU is taken once, and the weights' gradients go to
 // global memory once a CTA; one output per thread with its operands and SiLUs from shared memory
 // and a CTA's atomics per 32 samples took 280 us (forward) and 617 us (training) for 100 000
-// samples, this 46 and 190 us (with the loss one by one; 76 us of it went with half of that).
+// samples, this 46 and 112 us.  The loss is summed like the gradient of b3, a thread's tiles first
+// (1e-6 of it off up to a million samples; half of the samples one by one in one FP32 sum: 114 us,
+// and 1e-5 off at 100 000, 3e-4 at a million).
 template <bool TRAIN>
 __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
     mlp_tile_kernel(const __nv_bfloat16* __restrict__ wb, const MlpNorm norm, const float* __restrict__ x,
@@ -133,7 +127,7 @@ __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
         S.w3[t] = bf(wb, MLP_OFF_W3 + t);
     }
     const float b3 = bf(wb, MLP_OFF_B3);
-    [[maybe_unused]] float gw2[4][4], gw1[4][I], gb1[4], gw3 = 0.0f, gb2 = 0.0f, gb3 = 0.0f;
+    [[maybe_unused]] float gw2[4][4], gw1[4][I], gb1[4], gw3 = 0.0f, gb2 = 0.0f, gb3 = 0.0f, loss = 0.0f;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         gb1[j] = 0.0f;
@@ -226,12 +220,7 @@ __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
             if constexpr (TRAIN) {
                 S.D[t] = d;
                 gb3 += d;
-                if (n > MLP_SERIAL_LOSS && t < 32) {
-                    if (t < ns) atomicAdd(&grad[MLP_NPARAM], e);
-                } else {
-                    for (int q = 1; q < 32; q <<= 1) e += __shfl_xor_sync(0xffffffffu, e, q);
-                    if ((t & 31) == 0) atomicAdd(&grad[MLP_NPARAM], e);
-                }
+                loss += e;
             }
         }
         __syncthreads();
@@ -310,8 +299,14 @@ __global__ void __launch_bounds__(256, TRAIN ? 2 : MLP_FORWARD_CTAS)
         atomicAdd(&grad[MLP_OFF_B2 + (t >> 2)], gb2);
     }
     if (t < TB) {
-        for (int d = 1; d < 32; d <<= 1) gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
-        if ((t & 31) == 0) atomicAdd(&grad[MLP_OFF_B3], gb3);
+        for (int d = 1; d < 32; d <<= 1) {
+            gb3 += __shfl_xor_sync(0xffffffffu, gb3, d);
+            loss += __shfl_xor_sync(0xffffffffu, loss, d);
+        }
+        if ((t & 31) == 0) {
+            atomicAdd(&grad[MLP_OFF_B3], gb3);
+            atomicAdd(&grad[MLP_NPARAM], loss);
+        }
     }
     __syncthreads();
     for (int k = t; k < MLP_GROUP; k += 256) {
