@@ -215,7 +215,8 @@ RG_API int rg_calc_accel(rg_ctx* ctx, rg_vec_t* a);
  * Autotuner (not in the reference): times every candidate launch shape of the force
  * evaluation in the current gravity mode on the current state (`reps` evaluations each,
  * CUDA events on the context's stream) and keeps the fastest.  FP64 mode: sinks per
- * pair-parallel CTA x the row-kernel source limit -- every candidate sums in the same
+ * tile (of the certified kernel, where the disk has blocks for it; in the astrocentric frame per
+ * pair-parallel CTA), then the row-kernel source limit -- every candidate sums in the same
  * order, so results stay bit-exact; mixed mode: first the row-kernel limit, then the mixed
  * kernel's sources per grid.y chunk (whole tiles of 256 sources: for each chunk count up to
  * 24 the smallest chunk that gives it and one tile less, so that the grid's last wave of
@@ -394,7 +395,7 @@ RG_API int rg_ens_kernel_count(rg_ens* ens, int64_t* n_kernels, int64_t* n_graph
 /* Tile-shape autotuner of the ensemble (no counterpart in the reference, which has one
  * launch shape per kernel): times one gravity evaluation of every disk for each candidate
  * shape of the current gravity mode (`reps` evaluations each, CUDA events on the ensemble's
- * stream) and keeps the fastest.  FP64 mode: sinks per pair-parallel CTA x the row-kernel
+ * stream) and keeps the fastest.  FP64 mode: sinks per certified tile x the row-kernel
  * source limit -- every candidate sums in the reference's order, so results stay bit-exact;
  * mixed mode: sources per few-sink CTA -- for disks of a few heavy bodies and many light
  * ones, the light bodies per CTA of the symmetric heavy-light kernel, about, in whole waves

@@ -109,7 +109,7 @@ struct rg_ctx {
     int close_encounter = 0, inner_steps = 1, event_time_mode = RG_EVENT_TIME_CPU;
     double hill_factor = 0.0;
     int gravity_mode = RG_GRAVITY_FP64;
-    int pairpar_S = 16;
+    int pairpar_S = 16;  // sinks of a certified tile; astrocentric frame: of a pair-parallel CTA
     int rowseq_max_src = 64;
     int mixed_chunk_src = 0;  // sources per grid.y chunk of the mixed kernel, a multiple of
                               // MIXED_SOURCE_TILE (0: from the SM count)
@@ -1695,7 +1695,7 @@ int rg_device_count(void)
     return n;
 }
 
-// The default sinks per pair-parallel tile.  Barycentric frame: a tile's sinks are shared out
+// The default sinks per tile.  Barycentric frame: a certified tile's sinks are shared out
 // over independent warps (gravity_cert.cu), so only the last tile's unused warps depend on it.
 // Astrocentric frame: every CTA of the block runs all of its sources, so a launch takes (waves of
 // resident CTAs) x (one CTA's time, proportional to S); the S of the candidate set with the
@@ -2204,12 +2204,18 @@ static int autotune_impl(rg_ctx* c, int reps, rg_tune_t* out)
         for (int k : ks) cand.push_back({best.S, best.rowseq, k * MIXED_SOURCE_TILE});
         run(cand);
     } else {
-        // sinks per pair-parallel CTA (the astrocentric kernel has 8, 16 and 32), then the
-        // row-kernel source limit at the best of them
+        // sinks per certified tile (astrocentric frame: per pair-parallel CTA, 8, 16 or 32), then the
+        // row-kernel source limit at the best of them; a plan without certified tiles is the same for
+        // all of them, and timing it would choose by chance
         std::vector<int> ss = {8, 16, 32};
         if (c->frame != RG_FRAME_ASTRO) ss = {8, 12, 16, 18, 24, 32, 36};
+        bool shaped = c->frame == RG_FRAME_ASTRO;
+        for (const auto& gr : c->plan[0]) shaped = shaped || gr.kind == GROUP_CERT;
         for (int S : ss) cand.push_back({S, c->rowseq_max_src, c->mixed_chunk_src});
-        run(cand);
+        if (shaped)
+            run(cand);
+        else
+            n_cand += (int)cand.size();
         cand.clear();
         for (int r : rows) cand.push_back({best.S, r, c->mixed_chunk_src});
         run(cand);

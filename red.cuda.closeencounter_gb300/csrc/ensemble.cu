@@ -802,8 +802,8 @@ struct rg_ens {
     int n_sys = 0;
     int cap = 0;
     int device = 0, n_sm = 152;
-    // gravity launch shapes (rg_ens_autotune): row-kernel source limit, sinks per FP64
-    // pair-parallel CTA, sources per few-sink CTA (0: automatic)
+    // gravity launch shapes (rg_ens_autotune): row-kernel source limit, sinks per certified FP64
+    // tile, sources per few-sink CTA (0: automatic)
     int rowseq_max_src = 64, pairpar_S = 16, few_chunk = 0;
     int pairpar_sinks = 8;  // of a pair-parallel CTA
     std::vector<int> base, ntot;
@@ -2555,7 +2555,8 @@ static int time_ens_evaluations(rg_ens* e, int reps, double* ms)
     return RG_OK;
 }
 
-// the ensemble's tile shapes, timed on its own disks: FP64 mode sinks per pair-parallel CTA x
+// the ensemble's tile shapes, timed on its own disks: FP64 mode sinks per certified tile (where the plan
+// has such tiles: it is the same for all of them otherwise, and timing would choose by chance) x
 // the row-kernel source limit (each candidate sums in the reference's order: results stay
 // bit-exact), mixed mode sources per few-sink CTA x the row-kernel limit
 static int ens_autotune_impl(rg_ens* e, int reps, rg_tune_t* out)
@@ -2588,6 +2589,9 @@ static int ens_autotune_impl(rg_ens* e, int reps, rg_tune_t* out)
         e->few_chunk = sh.chunk;
         build_gravity_plan(e);
         rc = upload_plans(e);
+        bool shaped = e->gravity_mode == RG_GRAVITY_MIXED || sh.S == before.S;
+        for (const auto& gr : e->plan[0]) shaped = shaped || gr.kind == GROUP_CERT;
+        if (!shaped) continue;
         double ms = 0.0;
         if (!rc) rc = time_ens_evaluations(e, reps, &ms);
         if (!rc && ms < best_ms) {

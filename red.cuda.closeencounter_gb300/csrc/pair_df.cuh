@@ -93,7 +93,7 @@ __device__ __forceinline__ void exact_event_tests(const GravArgs& g, const Tile&
 //
 // The pairs whose terms need more than FP32 accuracy -- sinks against the star and giant
 // planets, and the star and giants' own rows -- would cost GB300 its scarce FP64 issue
-// (grav_fp64_rowseq and the few-sink kernels spend about 35 FP64 operations per pair).
+// (grav_fp64_rowseq and grav_fp64_rows spend about 35 FP64 operations per pair).
 // Here they run on the FP32 pipes in unevaluated sums of two floats (hi + lo, about 44
 // significant bits), built from the error-free transformations two-sum (Knuth) and
 // two-product by FMA, with the double-double addition and multiplication of Hida, Li and
