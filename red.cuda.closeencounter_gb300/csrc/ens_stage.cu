@@ -7,9 +7,9 @@
 // issue) with HBM idle.  Here warps in one phase run beside warps in the other, the stage positions
 // stay in registers instead of going through memory (24 bytes written and read a body), and a stage
 // has one launch, one prologue and one tail.  Measured: 128 attempts of 256 disks (1.1 million
-// bodies) 238 -> 215 ms, with the elements loaded when used 227 ms; attempts of eight disks of 512
-// bodies, all latency, 30 % more a second.  Now issue bounds it (65 % of cycles; six stage vectors
-// and the pairs are 88 million warp instructions).
+// bodies) 238 -> 215 ms (267 -> 240 ms with the disks' states read), with the elements loaded when
+// used 227 ms; attempts of eight disks of 512 bodies, all latency, 30 % more a second.  Now issue
+// bounds it (65 % of cycles; six stage vectors and the pairs are 88 million warp instructions).
 #include <atomic>
 #include <string>
 

@@ -47,8 +47,9 @@ int set_error(int code, const std::string& msg);
 // S sets the number of CTAs, ceil(sinks / S): the tuner picks the S whose grid fills the last
 // wave of resident CTAs best, since every CTA of a block runs the same sources and so takes the
 // same time.  In the barycentric frame the plan takes the S of the least waves x steps (PairparSinks):
-// 5000 / 20 000 sinks of 65 sources 14 / 49 us, a CTA per row 77 / 287 us, certified 41 / 70 us;
-// an RKF7(8) attempt of 64 / 256 disks of 103 / 73 bodies 529 / 963 us, in rows 1625 / 4095 us.
+// an evaluation of 65 massive bodies and 5000 / 20 000 test particles 23 / 57 us, their rows a CTA each
+// 85 / 295 us, certified 68 / 97 us; an RKF7(8) attempt of 64 / 256 disks of 103 / 73 bodies 529 / 963
+// us, in rows 1625 / 4095 us.
 template <int S, int STRIDE, bool ASTRO>
 __global__ void __launch_bounds__(S * STRIDE, RG_PAIRPAR_RESIDENT) grav_fp64_pairpar(GravArgs g)
 {

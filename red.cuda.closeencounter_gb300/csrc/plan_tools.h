@@ -19,9 +19,9 @@ namespace redgb {
 // GB300: rows 18 / 55 / 85 / 101 us, certified 48 / 88 / 99 / 109 us; of 1700 and 2000, before the
 // rows' last gain of a tenth, rows 146 / 195 us, certified 124 / 149 us.  Wide, shallow ones by their
 // rows: blocks of 65 / 103 / 203 / 403 sources cost the same in rows and pair by pair at some 600 /
-// 700 / 1000 / 1600 sinks (5000 sinks of 65: 77 us in rows, 14 pair by pair, 41 certified), and are
-// certified from some 100 000 / 16 000 / 5000 / 2000 sinks on (20 000 of 203: 165 us pair by pair,
-// 105 certified).
+// 700 / 1000 / 1600 sinks (an evaluation of 65 massive bodies and 5000 test particles: 85 us in rows, 23
+// pair by pair, 68 certified), and are certified from some 100 000 / 16 000 / 5000 / 2000 sinks on
+// (203 and 20 000: 189 us pair by pair, 117 certified).
 enum Fp64Form { FP64_FORM_ROWS, FP64_FORM_PAIRPAR, FP64_FORM_CERT };
 constexpr int64_t FP64_ROW_PAIRS = 2250000;
 inline bool fp64_wide(int64_t rows, int64_t pairs)  // rows > 400 + 2.8 sources
@@ -36,9 +36,9 @@ inline Fp64Form fp64_block_form(int64_t rows, int64_t pairs)
 
 // The sinks S of a pair-parallel CTA for the blocks added: 256 threads take four terms each of S x
 // 1024 / S pairs at a time, `resident` CTAs on each of n_sm SMs.  The S of the least waves x steps (a
-// CTA starts and sums for as long as two steps of terms take; half a wave's rounding counts: of 203
-// sources, 2000 sinks take 28 us with 8 and 44 with 16, 5000 take 72 and 63; 64 disks of 103 bodies
-// 565 us an attempt with 8, 529 with 16, 661 with 32).
+// CTA starts and sums for as long as two steps of terms take; half a wave's rounding counts: an
+// evaluation of 203 massive bodies and 2000 test particles takes 39 us with 8 and 54 with 16, with
+// 5000 82 and 73; 64 disks of 103 bodies 565 us an attempt with 8, 529 with 16, 661 with 32).
 struct PairparSinks {
     static constexpr int S[4] = {4, 8, 16, 32};
     double ctas[4] = {}, steps[4] = {};
