@@ -1790,7 +1790,7 @@ static int create_impl(const rg_counts_t* n, const rg_vec_t* r, const rg_vec_t* 
     chk(dalloc(&c->cert.rows, (size_t)(8 * c->cert.stride)));
     chk(dalloc(&c->cert.scale, 8));
     chk(dalloc(&c->cert.list, nt));
-    chk(dalloc(&c->cert.n_list, 1));
+    chk(dalloc(&c->cert.n_list, CERT_COUNTERS));
     chk(dalloc(&c->d_rf, nt));
     chk(dalloc(&c->d_smax, SCREEN_MAX_WORDS));
     chk(dalloc(&c->d_screen_slot, nt));

@@ -1888,7 +1888,7 @@ int create_impl(int n_sys, const rg_counts_t* counts, const rg_vec_t* r, const r
     chk(dalloc(&e->cert.rows, certified ? (size_t)(8 * e->cert.stride) : 1));
     chk(dalloc(&e->cert.scale, 8 * ns));
     chk(dalloc(&e->cert.list, certified ? nt : 1));
-    chk(dalloc(&e->cert.n_list, 1));
+    chk(dalloc(&e->cert.n_list, CERT_COUNTERS));
     chk(dalloc(&e->d_rf, nt));
     chk(dalloc(&e->d_mass_f2, nt));
     chk(dalloc(&e->d_smax, (size_t)SCREEN_MAX_WORDS * ns));

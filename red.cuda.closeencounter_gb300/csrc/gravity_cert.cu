@@ -101,7 +101,7 @@ struct alignas(16) CertSmem {  // rows are read and copied to 16 bytes at a time
     double acc[3][SW];
     long long part[NQ][3][SW];               // a lane's sum of quanta
     float bnd[NQ][3][SW];                    // and of their magnitudes (infinite: it has no quanta)
-    float sig[3][SW];                        // 2^-16 / Q; 0 for acc = 0; NaN: every pair exactly
+    float sig[3][SW];                        // 2^-16 / Q; 0 for acc = 0 and for a sum left to the row kernel
     unsigned short fitem[32];
 };
 
@@ -112,7 +112,7 @@ __device__ __forceinline__ float pow2f(int e)  // e in [-126, 127]
 
 __device__ __forceinline__ int expo(float v) { return (int)((__float_as_uint(v) >> 23) & 0xffu) - 127; }
 
-// 2^-16 / Q of a running sum: 0 for zero, NaN outside [2^-40, 2^120]
+// 2^-16 / Q of a running sum: 0 for zero, NaN outside [2^-40, 2^120] and for one that is not finite
 __device__ __forceinline__ float sigma_of(double acc)
 {
     const int ea = (int)((xf::dbits(acc) >> 52) & 0x7ff);
@@ -319,7 +319,7 @@ struct CertPrepArgs {
     int screen;
     float* rows;
     long long stride;
-    unsigned int* n_list;   // rows left to grav_fp64_rows: none yet
+    unsigned int* n_list;   // counts of rows left to grav_fp64_rows: none yet
     float* scale;           // 8 per system: max |x|, |y|; max |z|; the screens' maxima of R, m, rho;
                             // bits: components in which every displacement is zero
 };
@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
     const long long sys_of = cta / a.blocks;
     if (sys_of >= a.n_sys) return;
     const int sys = (int)sys_of, block = (int)(cta - sys_of * a.blocks);
-    if (cta == 0 && threadIdx.x == 0) *a.n_list = 0u;
+    if (cta == 0 && threadIdx.x < CERT_COUNTERS) a.n_list[threadIdx.x] = 0u;
     const int b0 = a.sys_base ? a.sys_base[sys] : 0, b1 = b0 + (a.sys_base ? a.sys_n[sys] : a.n);
     const int j = b0 + block * PREP_NT + threadIdx.x;
     if (b0 + block * PREP_NT >= b1 || (a.sys_active && !a.sys_active[sys])) return;
@@ -461,7 +461,13 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 // has left its binade in four epochs, the sink goes to a list of rows, the component is dropped
 // here, and grav_fp64_rows adds it from exact terms.  A sink outside the grid goes there whole, with
 // its event tests: its exact pairs in one warp would be the last thing running (one body at 100 AU
-// in a disk of 8003 bodies with collisions on: an RKF7(8) attempt 21.7 ms, 8.9 without it).
+// in a disk of 8003 bodies with collisions on: an RKF7(8) attempt 21.7 ms, 8.9 without it).  So does
+// a sink with an eighth of its pairs flagged that no failing component explains (sources outside the
+// grid, wide screens), whose exact pairs cost eleven times the row kernel's, and so do all, once
+// three quarters of the sinks begun have rows in the list (a disk's row costs three of its sinks
+// here); and a sink whose sums are all left to the row kernel is done here.  An RK4 step of 8003
+// bodies with collisions on, of them 10 / 30 % out to thousands of AU 22.2 / 30.3 -> 9.8 / 10.6 ms, 10 %
+// above an otherwise flat disk 29.8 -> 11.8 ms (every pair on the FP64 pipe: 9.7 ms).
 template <int SW, bool SCREEN>
 __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     grav_fp64_cert(GravArgs g, CertRows cr)
@@ -469,7 +475,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     using Sm = CertSmem<SW>;
     static_assert(sizeof(Sm) % 16 == 0 && Sm::PITCH % 4 == 0 && HEAD % 4 == 0, "16-byte copies");
     constexpr int NQ = Sm::NQ, PITCH = Sm::PITCH, SLICE = Sm::SLICE, PART = Sm::PART, EPOCH = SLICE * NQ;
-    constexpr unsigned ALL = 0xffffffffu;
+    constexpr unsigned ALL = 0xffffffffu, SINKS = (1u << SW) - 1u;
     __shared__ __align__(16) Sm smem[CERT_WARPS];
     Sm& M = smem[threadIdx.x >> 5];
 
@@ -496,6 +502,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     const float* const base = cr.rows + cert_row(tile.base, tile.sys) - tile.base;  // [j]: body j
     CertSink k;
     bool outside;  // the grid: left to the row kernel whole, event tests and all
+    if (lane == 0) atomicAdd(cr.n_list + 1, (unsigned)__popc(act & SINKS));
     {
         const float* p = base + (active ? i : tile.base);
         const float lim = pow2f(max(-50, expo(cr.scale[8 * tile.sys])) + 1);
@@ -592,7 +599,12 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
         __syncwarp();
         if (owner) {
             M.acc[c][s] = acc;
-            M.sig[c][s] = (act >> s & 1) && !deferred ? sigma_of(acc) : 0.0f;
+            float sigma = (act >> s & 1) && !deferred ? sigma_of(acc) : 0.0f;
+            if (sigma != sigma) {  // out of range (all but zero, as a coplanar body's z): every pair would be exact
+                deferred = true;
+                sigma = 0.0f;
+            }
+            M.sig[c][s] = sigma;
         }
         __syncwarp();
     };
@@ -629,20 +641,25 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     };
     fetch(j0, 0);
     fetch(j0, 1);
-    int n_redo = 0;
-    unsigned live = act & ~__ballot_sync(ALL, outside);  // sinks with sums left here (or events to find)
+    int n_redo = 0, n_exact = 0;  // n_exact: this lane's flagged pairs that no failing component explains
+    int tests = outside ? j_head : tile.src_end;  // the first source whose event tests are the row kernel's
+    unsigned live = act & ~__ballot_sync(ALL, outside) & SINKS;  // sinks with sums left here (or events to find)
+    unsigned listed = act & SINKS & ~live;                       // sinks with a row in the list
     for (; j0 < tile.src_end; j0 += EPOCH) {
         const int nj = min(EPOCH, tile.src_end - j0);
         const int sl = nj == EPOCH ? SLICE : ((nj + NQ * 4 - 1) / (NQ * 4)) * 4;
         const int cnt = max(0, min(sl, nj - q * sl));
+        const int passed = j0 - j_head;
+        const bool look = passed < 8 * EPOCH || passed % (16 * EPOCH) == 0;  // whether the sinks had better go whole
+        unsigned begun = 0u, rows = 0u;
+        if (look && lane == 0) begun = __ldcg(cr.n_list + 1), rows = __ldcg(cr.n_list + 2);
         CertSum sum{0u, 0u, 0u, 0u, 0u, 0u, 0.0f};
         unsigned flags = 0u;
         const float sx = M.sig[0][s], sy = M.sig[1][s], sz = M.sig[2][s];
         k.sx = f2_dup(sx);
         k.sy = f2_dup(sy);
         k.sz = f2_dup(sz);
-        float cut = SCREEN && j0 < i ? event_cut : MIN_R2;
-        if (sx != sx || sy != sy || sz != sz) cut = 3.0e38f;
+        const float cut = SCREEN && j0 < i ? event_cut : MIN_R2;
         int n_done = 0;
 #pragma unroll 1
         for (int h = 0; h < SLICE / PART; h++) {
@@ -733,6 +750,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
                 by += bad & 2 ? inf : __ll2float_ru(ry < 0 ? -ry : ry);
                 bz += bad & 4 ? inf : __ll2float_ru(rz < 0 ? -rz : rz);
                 fail += (bad >> 3 & 1u) | (bad >> 4 & 1u) << 10 | (bad >> 5 & 1u) << 20;
+                n_exact += bad >> 3 == 0u;
             }
             __syncwarp();  // the round's lists are read before the next round writes them
         }
@@ -756,15 +774,26 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
             ok = accept(acc, total, bound) || (acc == 0.0 && (flat >> c & 1) && bound < 1.0e30f);
         }
         for (int off = SW; off < 32; off <<= 1) fail += __shfl_xor_sync(ALL, fail, off);
+        bool whole = false;
+        if (look) {
+            int n = n_exact;
+            for (int off = SW; off < 32; off <<= 1) n += __shfl_xor_sync(ALL, n, off);
+            const bool many = __any_sync(ALL, begun >= 512u && 4ull * rows > 3ull * begun);  // (by every lane)
+            whole = many || (n > 32 && 8 * n > passed + nj);
+        }
         if (owner && !deferred && (act >> s & 1)) {
-            n_redo += !ok;
-            deferred = deferred || (int)(fail >> (10 * c) & 1023u) * 8 > nj || n_redo >= 4;
+            n_redo += ok ? 0 : (acc == 0.0 ? 4 : 1);  // (a sum that is zero so far will hover)
+            deferred = deferred || whole || (int)(fail >> (10 * c) & 1023u) * 8 > nj || n_redo >= 4;
             ok = ok || deferred;
         }
         // sums (bit c SW + s) whose epoch is taken slice by slice
         const unsigned redo = __ballot_sync(ALL, !ok);
         const unsigned gone = __ballot_sync(ALL, deferred);
-        if (!SCREEN) live &= ~(gone & gone >> SW & gone >> 2 * SW);
+        const unsigned done = gone & gone >> SW & gone >> 2 * SW & live, some = (gone | gone >> SW | gone >> 2 * SW) & live;
+        if (done >> s & 1u) tests = min(j0 + EPOCH, tile.src_end);
+        live &= ~done;
+        if (lane == 0 && (some & ~listed)) atomicAdd(cr.n_list + 2, (unsigned)__popc(some & ~listed));
+        listed |= some;
         // the others slice by slice: its quanta while the sum stays in the epoch's binade, else
         // its exact terms added in order
         for (unsigned left_sums = redo; left_sums; left_sums &= left_sums - 1) {
@@ -780,6 +809,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
             }
             if (lane == w) acc = a;
         }
+        if (!live) break;  // (uniform)
         publish();
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -793,8 +823,8 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
         if (mask) {
             Tile row = tile;
             row.sink_begin = i;
-            row.sink_end = outside ? j_head : tile.src_end;
-            row.part = mask;
+            row.sink_end = tests;
+            row.part = mask | (int)((__float_as_uint(event_cut) + 8u) & ~7u);
             cr.list[atomicAdd(cr.n_list, 1u)] = row;
         }
     }

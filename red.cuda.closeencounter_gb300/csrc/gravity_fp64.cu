@@ -232,17 +232,19 @@ struct RowSmem {
 };
 
 // the event tests of a listed row's body with the sources from sink_end on (a pair's tests are its later
-// body's), by a CTA; out of the row kernel's own code
+// body's), by a CTA: for the few rows with a pair that may pass, out of the row kernel's own code
 __device__ __noinline__ void row_events(const GravArgs& g, const Tile* row)
 {
     const Tile tile = *row;
     const int i = tile.sink_begin;
     if (!(0 < g.id[i])) return;
+    const double xi = g.px[i], yi = g.py[i], zi = g.pz[i], cut = __int_as_float(tile.part & ~7);
     for (int j = tile.sink_end + (int)threadIdx.x; j < min(i, tile.src_end); j += blockDim.x) {
+        const double dx = g.px[j] - xi, dy = g.py[j] - yi, dz = g.pz[j] - zi;
         PairOut o;
-        if (0 <= g.id[j])
-            pair_term(g, tile, i, j, g.px[i], g.py[i], g.pz[i], g.radius[i], g.mass[i], g.hill ? g.rho[i] : 0.0, g.px[j],
-                      g.py[j], g.pz[j], g.mass[j], g.radius[j], g.hill ? g.rho[j] : 0.0, o);
+        if (!(dx * dx + dy * dy + dz * dz >= cut) && 0 <= g.id[j])
+            pair_term(g, tile, i, j, xi, yi, zi, g.radius[i], g.mass[i], g.hill ? g.rho[i] : 0.0, g.px[j], g.py[j],
+                      g.pz[j], g.mass[j], g.radius[j], g.hill ? g.rho[j] : 0.0, o);
     }
 }
 
@@ -263,7 +265,7 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
     for (int row = blockIdx.x; row < n_rows; row += gridDim.x) {
         const Tile tile = LIST ? list[row] : g.tiles[row];
         if (g.sys_active && !g.sys_active[tile.sys]) continue;
-        const int comps = LIST ? tile.part : 7;
+        const int comps = LIST ? tile.part & 7 : 7;
         const int i = tile.sink_begin;
         const bool active = 0 < g.id[i];
         const double xi = g.px[i], yi = g.py[i], zi = g.pz[i];
@@ -272,6 +274,11 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
         const int n = tile.src_end - tile.src_begin;
         const int chunks = (n + ROW_CHUNK - 1) / ROW_CHUNK;
         const bool adds = comp < 3 && (comps >> comp & 1);
+        // a listed row's event tests: the upper word of the r^2 that none passes, -1 where it has none to make
+        [[maybe_unused]] const int cut = LIST && tile.sink_end < min(i, tile.src_end) && (g.record || g.hill)
+                                             ? __double2hiint((double)__int_as_float(tile.part & ~7))
+                                             : -1;
+        [[maybe_unused]] bool candidate = false;
         for (int c = 0; c <= chunks; c++) {
             if (c < chunks && (c == 0 || comp >= 3)) {  // terms of chunk c (the first one: by every warp)
                 const int q0 = c * ROW_CHUNK, m = min(ROW_CHUNK, n - q0);
@@ -280,10 +287,11 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
                 for (int q = (warp - w0) * 32 + lane; q < m; q += 32 * nw) {
                     const int j = tile.src_begin + q0 + q;
                     const double xj = g.px[j], yj = g.py[j], zj = g.pz[j], mj = g.mass[j];
-                    PairOut o{0.0, 0.0, 0.0};
+                    PairOut o{0.0, 0.0, 0.0, 1e300};
                     if (active && j != i && 0 <= g.id[j])
                         pair_term<!LIST>(g, tile, i, j, xi, yi, zi, Ri, mi, rhoi, xj, yj, zj, mj, LIST ? 0.0 : g.radius[j],
                                          !LIST && g.hill ? g.rho[j] : 0.0, o);
+                    if (LIST) candidate = candidate || (j >= tile.sink_end && j < i && __double2hiint(o.r2) <= cut);
                     const int at = q / seg * pitch + q % seg;
                     M.term[c & 1][0][at] = o.tx;
                     M.term[c & 1][1][at] = o.ty;
@@ -302,7 +310,7 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
             __syncthreads();
         }
         if (adds && (int)threadIdx.x == LANES * comp) (comp == 0 ? g.ax : comp == 1 ? g.ay : g.az)[i] = acc;
-        if (LIST && tile.sink_end < min(i, tile.src_end) && (g.record || g.hill)) row_events(g, list + row);
+        if (LIST && cut >= 0 && __syncthreads_or(candidate)) row_events(g, list + row);
     }
 }
 

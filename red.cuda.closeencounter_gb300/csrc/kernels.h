@@ -84,10 +84,12 @@ struct CertRows {
     float* rows;       // 8 FP32 rows of `stride` (cert_stride)
     long long stride;
     float* scale;      // 8 per system
-    Tile* list;        // rows left over: one sink each, part = its components (bits), sink_end = the first
-                       // source it is to test for events (src_end: none); one slot per body
-    unsigned int* n_list;
+    // rows left over: one sink each; part: its components (bits 0 to 2) and the bits of the r^2 from which on no
+    // event test passes; sink_end: the first source it is to test (src_end: none).  One slot per body
+    Tile* list;
+    unsigned int* n_list;  // CERT_COUNTERS: the list's length, sinks begun, sinks with a row in the list
 };
+constexpr int CERT_COUNTERS = 3;
 long long cert_stride(int n, int n_sys);
 int launch_cert_prep(const GravArgs& g, const int* sys_base, const int* sys_n, int n_sys, int max_n, const CertRows& cr,
                      cudaStream_t st);

@@ -9,6 +9,7 @@ namespace redgb {
 
 struct PairOut {
     double tx, ty, tz;
+    double r2;  // set by pair_term
 };
 
 // the event tests of a pair at distance d and their records
@@ -66,7 +67,7 @@ __device__ __forceinline__ void pair_term(const GravArgs& g, const Tile& tile, i
     const double dx = xj - xi;
     const double dy = yj - yi;
     const double dz = zj - zi;
-    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double r2 = o.r2 = dx * dx + dy * dy + dz * dz;
     const double d = PIPE ? __dsqrt_rn(r2) : rn_sqrt(r2);  // rn_*: on the integer pipes (exact_fp64.h)
     const double w = PIPE ? __ddiv_rn(mj, d * r2) : rn_div(mj, d * r2);
     o.tx = w * dx;

@@ -66,7 +66,7 @@ int main()
     cr.stride = cert_stride(n, n_sys);
     cr.rows = up(std::vector<float>(8 * cr.stride));
     cr.scale = up(std::vector<float>(8 * n_sys));
-    cr.n_list = up(std::vector<unsigned int>(1, 7u));
+    cr.n_list = up(std::vector<unsigned int>(CERT_COUNTERS, 7u));
     if (launch_cert_prep(g, up(base), up(count), n_sys, 2500, cr, nullptr)) return 2;
     std::vector<float> scale(8 * n_sys);
     unsigned int n_list = 1;
