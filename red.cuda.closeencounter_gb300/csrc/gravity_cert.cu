@@ -464,8 +464,8 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 // in a disk of 8003 bodies with collisions on: an RKF7(8) attempt 21.7 ms, 8.9 without it).  So does
 // a sink with an eighth of its pairs flagged that no failing component explains (sources outside the
 // grid, wide screens), whose exact pairs cost eleven times the row kernel's, and so do all, once
-// three quarters of the sinks begun have rows in the list (a disk's row costs three of its sinks
-// here); and a sink whose sums are all left to the row kernel is done here.  An RK4 step of 8003
+// three quarters of the sinks begun have rows in the list (a row costs what three or four
+// sinks do here); and a sink whose sums are all left to the row kernel is done here.  An RK4 step of 8003
 // bodies with collisions on, of them 10 / 30 % out to thousands of AU 22.2 / 30.3 -> 9.8 / 10.6 ms, 10 %
 // above an otherwise flat disk 29.8 -> 11.8 ms (every pair on the FP64 pipe: 9.7 ms).
 template <int SW, bool SCREEN>

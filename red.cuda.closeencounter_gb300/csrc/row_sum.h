@@ -179,6 +179,22 @@ XF_HD bool row_diff(uint64_t x, uint64_t y, int* d, int64_t limit = MAX_OFF)
 constexpr int ROW_SEG_MAX = 36;  // terms per lane and call
 constexpr int ROW_CTA_WARPS = 16;  // most warps of cta_row_sum
 
+// the plain chain: acc + T_0 + ... + T_{m-1}, by every lane alike
+__device__ __forceinline__ double row_chain(double acc, const double* T, int seg, int pitch, int m)
+{
+    for (int l = 0; l * seg < m; l++) {
+        const double* const t = T + l * pitch;
+        const int n = min(seg, m - l * seg);
+#pragma unroll 4
+        for (int k = 0; k < n; k++) acc = __dadd_rn(acc, t[k]);
+    }
+    return acc;
+}
+// Whether it is shorter than adding `lanes` segments again: each costs its additions and some ten more.
+// (Sums through zero at every other term, as of bodies in antipodal pairs: an RKF7(8) attempt of 1003 such
+// bodies 1770 us with every lane added again, 700 so.)
+__device__ __forceinline__ bool row_chain_pays(int lanes, int seg, int m) { return lanes * (seg + 10) > m; }
+
 // acc + T_0 + ... + T_{m-1}, rounded after every addition in that order, m <= 32 seg,
 // seg <= ROW_SEG_MAX: term e is at T[e / seg * pitch + e % seg].  Every lane of the warp calls
 // this with the same arguments and returns the sum.  codes: 32 ROW_SEG_MAX entries of shared
@@ -245,6 +261,7 @@ __device__ __forceinline__ double warp_row_sum(double acc, const double* T, int 
     const bool slow = hard || loose || P >= LIM || P <= -LIM;
     unsigned todo = __ballot_sync(ALL, lane > 0 && (nc > 0 || slow));
     unsigned slows = __ballot_sync(ALL, slow);
+    if (row_chain_pays(__popc(slows & ~1u), seg, m)) return row_chain(acc, T, seg, pitch, m);
     uint64_t tend = end;  // of a lane that has been through the loop below: its true end
     bool done = lane == 0;
     int off = 0;  // offset of a lane = P + off, for the lanes after the last one done
@@ -500,6 +517,8 @@ __device__ __forceinline__ double group_row_sum(const RowGroup& grp, double acc,
         double sum = acc;
         if (most < LIM)
             sum = __longlong_as_double((long long)rs::row_shift(S.last, off + S.last_in));
+        else if (row_chain_pays(n_hard, seg, m))
+            sum = row_chain(sum, T, seg, pitch, m);
         else  // (the codes' space is free: they are not used)
             for (int w = 0; w < W && w * 32 * seg < m; w++)
                 sum = warp_row_sum(sum, T + w * 32 * pitch, seg, pitch, min(m - w * 32 * seg, 32 * seg), codes);
