@@ -232,8 +232,8 @@ struct RowSmem {
 };
 
 // the event tests of a listed row's body with the sources from sink_end on (a pair's tests are its later
-// body's), by a CTA: for the few rows with a pair that may pass, out of the row kernel's own code
-__device__ __noinline__ void row_events(const GravArgs& g, const Tile* row)
+// body's), by a CTA: for the few rows with a pair that may pass
+__device__ __forceinline__ void row_events(const GravArgs& g, const Tile* row)
 {
     const Tile tile = *row;
     const int i = tile.sink_begin;
@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32 * RowShape<LIST, TERMS>::WARPS, RowShape<LI
                     if (active && j != i && 0 <= g.id[j])
                         pair_term<!LIST>(g, tile, i, j, xi, yi, zi, Ri, mi, rhoi, xj, yj, zj, mj, LIST ? 0.0 : g.radius[j],
                                          !LIST && g.hill ? g.rho[j] : 0.0, o);
-                    if (LIST) candidate = candidate || (j >= tile.sink_end && j < i && __double2hiint(o.r2) <= cut);
+                    if (LIST) candidate = candidate | (__double2hiint(o.r2) <= cut);
                     const int at = q / seg * pitch + q % seg;
                     M.term[c & 1][0][at] = o.tx;
                     M.term[c & 1][1][at] = o.ty;
