@@ -805,7 +805,7 @@ struct rg_ens {
     // gravity launch shapes (rg_ens_autotune): row-kernel source limit, sinks per certified FP64
     // tile, sources per few-sink CTA (0: automatic)
     int rowseq_max_src = 64, pairpar_S = 16, few_chunk = 0;
-    int pairpar_sinks = 8;  // of a pair-parallel CTA
+    int pairpar_sinks[2] = {8, 8};  // of a pair-parallel CTA: blocks of many sinks, of few
     std::vector<int> base, ntot;
     std::vector<std::array<int, 7>> cnt;
     std::vector<rg_param_t> p;
@@ -972,7 +972,8 @@ enum {
     GROUP_DF_FEW = 5,
     GROUP_DF_SYM = 6,  // heavy-light pairs once for both rows, with its systems' heavy rows
     GROUP_PAIRPAR = 7,
-    GROUP_KINDS = 8
+    GROUP_PAIRPAR_FEW = 8,  // of few sinks a system, fewer sinks a CTA
+    GROUP_KINDS = 9
 };
 constexpr int ENS_SYM_CHUNK = 2048;  // light bodies per symmetric tile about, unless tuned
 
@@ -1107,9 +1108,8 @@ void build_gravity_plan(rg_ens* e)
         for (size_t k = 0; k < sym_systems.size(); k++) sym_parts[sym_systems[k].sys] = parts[k];
     }
     // The FP64 form of the blocks with many sources, all disks' together: of each kind of block those with
-    // many sinks (without the wide and shallow ones all or none certified), and [3] the rows of few
-    // sinks: blocks of them, and the heavy rows beside certified ones (their terms are as large as their
-    // sums, gravity_cert.cu)
+    // many sinks (all certified where one is), and [3] the rows of few sinks: blocks of them, and the heavy
+    // rows beside certified ones (their terms are as large as their sums, gravity_cert.cu)
     const auto block_of = [&](int s, int k, int64_t* sinks, int64_t* sources) {
         const int64_t nsi = e->n_si(s), nm = e->n_massive(s);
         *sinks = k == 0 ? nsi : (k == 1 ? nm - nsi : e->ntot[s] - nm);
@@ -1133,8 +1133,11 @@ void build_gravity_plan(rg_ens* e)
         if (form[k] != FP64_FORM_PAIRPAR) rest += pairs[k];
         cert = cert || form[k] == FP64_FORM_CERT;
     }
+    // (where the certified kernel runs, more rows of it cost less than another kernel's launch: 12 disks of
+    // 303 massive bodies, 300 planetesimals and 300 test particles 1949 us an attempt, the planetesimals'
+    // block pair by pair 2429 us)
     for (int k = 0; k < 3; k++)
-        if (form[k] == FP64_FORM_ROWS && (cert || rest > FP64_ROW_PAIRS)) form[k] = FP64_FORM_CERT;
+        if (cert || (form[k] == FP64_FORM_ROWS && rest > FP64_ROW_PAIRS)) form[k] = FP64_FORM_CERT;
     for (int s = 0; s < e->n_sys; s++)
         if (block_of(s, 0, &ns, &nsrc) && ns > ENS_FEW_BLOCK && form[0] == FP64_FORM_CERT && heavy_of(s) <= ENS_FEW_BLOCK) {
             rows[3] += heavy_of(s);
@@ -1142,13 +1145,13 @@ void build_gravity_plan(rg_ens* e)
         }
     form[3] = fp64_wide(rows[3], pairs[3]) ? FP64_FORM_PAIRPAR : FP64_FORM_ROWS;
     // where the pair-parallel kernel runs, short rows are a few CTAs more of it (4 disks of 103 bodies
-    // and 2000 test particles: 1105 us an attempt with a launch for the rows, 991 without)
+    // and 2000 test particles: 1105 us an attempt with a launch for the rows, 885 to 991 without)
     if (std::find(form, form + 4, FP64_FORM_PAIRPAR) != form + 4)
         for (int k = 0; k < 4; k++)
             if (form[k] == FP64_FORM_ROWS && pairs[k] <= 256 * rows[k]) form[k] = FP64_FORM_PAIRPAR;
-    const int few_kind = form[3] == FP64_FORM_PAIRPAR ? GROUP_PAIRPAR : GROUP_FP64_ROWS;
-    std::vector<Tile> wide;  // the pair-parallel kernel's blocks, to be cut when all are known
-    PairparSinks sinks;
+    const int few_kind = form[3] == FP64_FORM_PAIRPAR ? GROUP_PAIRPAR_FEW : GROUP_FP64_ROWS;
+    std::vector<Tile> wide[2];  // the pair-parallel kernel's blocks (many sinks, few), to be cut when all are known
+    PairparSinks sinks[2];
     for (int s = 0; s < e->n_sys; s++) {
         const int b = e->base[s];
         const int nsi = e->n_si(s), nm = e->n_massive(s), nt = e->ntot[s];
@@ -1159,9 +1162,9 @@ void build_gravity_plan(rg_ens* e)
             int s0, s1, src1, block;
         } blks[3] = {{0, nsi, nm, 0}, {nsi, nm, nsi, 1}, {nm, nt, nm, 2}};
         auto add = [&](int mode, int kind, int s0, int s1, int src1, int block, int step) {
-            if (kind == GROUP_PAIRPAR && s0 < s1) {
-                wide.push_back(Tile{b + s0, b + s1, b, b + src1, s, b, block, 0});
-                sinks.add(s1 - s0, src1);
+            if ((kind == GROUP_PAIRPAR || kind == GROUP_PAIRPAR_FEW) && s0 < s1) {
+                wide[kind - GROUP_PAIRPAR].push_back(Tile{b + s0, b + s1, b, b + src1, s, b, block, 0});
+                sinks[kind - GROUP_PAIRPAR].add(s1 - s0, src1);
                 return;
             }
             for (int q = s0; q < s1; q += step) {
@@ -1193,15 +1196,17 @@ void build_gravity_plan(rg_ens* e)
             }
         }
     }
-    e->pairpar_sinks = sinks.best(RG_PAIRPAR_RESIDENT, e->n_sm);
-    for (const Tile& w : wide)
-        for (int q = w.sink_begin; q < w.sink_end; q += e->pairpar_sinks) {
-            Tile t = w;
-            t.sink_begin = q;
-            t.sink_end = std::min(q + e->pairpar_sinks, w.sink_end);
-            by[0][GROUP_PAIRPAR].push_back(t);
-            hv[0][GROUP_PAIRPAR].push_back(0);
-        }
+    for (int k = 0; k < 2; k++) {
+        const int S = e->pairpar_sinks[k] = sinks[k].best(RG_PAIRPAR_RESIDENT, e->n_sm);
+        for (const Tile& w : wide[k])
+            for (int q = w.sink_begin; q < w.sink_end; q += S) {
+                Tile t = w;
+                t.sink_begin = q;
+                t.sink_end = std::min(q + S, w.sink_end);
+                by[0][GROUP_PAIRPAR + k].push_back(t);
+                hv[0][GROUP_PAIRPAR + k].push_back(0);
+            }
+    }
     for (int mode = 0; mode < 2; mode++) {
         e->plan[mode].clear();
         for (int kind = 0; kind < GROUP_KINDS; kind++) {
@@ -1412,7 +1417,11 @@ int ens_gravity(rg_ens* e, const double* pos, const double* vel, double* acc, in
         g.tiles = e->d_tiles + gr.off;
         g.n_tiles = gr.n;
         switch (gr.kind) {
-        case GROUP_PAIRPAR: rc = launch_grav_fp64_pairpar(g, e->pairpar_sinks, e->st); e->n_kernels++; break;
+        case GROUP_PAIRPAR:
+        case GROUP_PAIRPAR_FEW:
+            rc = launch_grav_fp64_pairpar(g, e->pairpar_sinks[gr.kind - GROUP_PAIRPAR], e->st);
+            e->n_kernels++;
+            break;
         case GROUP_CERT:
             if (!split_done) {
                 rc = launch_cert_prep(g, e->d_base, e->d_ntot, e->n_sys, e->max_n, e->cert, e->st);

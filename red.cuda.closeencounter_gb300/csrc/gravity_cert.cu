@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     const float* const base = cr.rows + cert_row(tile.base, tile.sys) - tile.base;  // [j]: body j
     CertSink k;
     bool outside;  // the grid: left to the row kernel whole, event tests and all
-    if (lane == 0) atomicAdd(cr.n_list + 1, (unsigned)__popc(act & SINKS));
+    const bool counted = tile.src_end - tile.src_begin > 4 * EPOCH;  // rows long enough to learn from the others' fate
+    if (counted && lane == 0) atomicAdd(cr.n_list + 1, (unsigned)__popc(act & SINKS));
     {
         const float* p = base + (active ? i : tile.base);
         const float lim = pow2f(max(-50, expo(cr.scale[8 * tile.sys])) + 1);
@@ -652,7 +653,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
         const int passed = j0 - j_head;
         const bool look = passed < 8 * EPOCH || passed % (16 * EPOCH) == 0;  // whether the sinks had better go whole
         unsigned begun = 0u, rows = 0u;
-        if (look && lane == 0) begun = __ldcg(cr.n_list + 1), rows = __ldcg(cr.n_list + 2);
+        if (counted && look && lane == 0) begun = __ldcg(cr.n_list + 1), rows = __ldcg(cr.n_list + 2);
         CertSum sum{0u, 0u, 0u, 0u, 0u, 0u, 0.0f};
         unsigned flags = 0u;
         const float sx = M.sig[0][s], sy = M.sig[1][s], sz = M.sig[2][s];
@@ -792,7 +793,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
         const unsigned done = gone & gone >> SW & gone >> 2 * SW & live, some = (gone | gone >> SW | gone >> 2 * SW) & live;
         if (done >> s & 1u) tests = min(j0 + EPOCH, tile.src_end);
         live &= ~done;
-        if (lane == 0 && (some & ~listed)) atomicAdd(cr.n_list + 2, (unsigned)__popc(some & ~listed));
+        if (counted && lane == 0 && (some & ~listed)) atomicAdd(cr.n_list + 2, (unsigned)__popc(some & ~listed));
         listed |= some;
         // the others slice by slice: its quanta while the sum stays in the epoch's binade, else
         // its exact terms added in order

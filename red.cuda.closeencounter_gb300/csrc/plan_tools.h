@@ -18,25 +18,27 @@ namespace redgb {
 // Square blocks go by their pairs: self-interacting blocks of 400 / 1000 / 1300 / 1480 bodies on
 // GB300: rows 18 / 55 / 85 / 101 us, certified 48 / 88 / 99 / 109 us; of 1700 and 2000, before the
 // rows' last gain of a tenth, rows 146 / 195 us, certified 124 / 149 us.  Wide, shallow ones by their
-// rows: blocks of 65 / 103 / 203 / 403 sources cost the same in rows and pair by pair at some 600 /
-// 700 / 1000 / 1600 sinks (an evaluation of 65 massive bodies and 5000 test particles: 85 us in rows, 23
-// pair by pair, 68 certified), and are certified from some 100 000 / 16 000 / 5000 / 2000 sinks on
-// (203 and 20 000: 189 us pair by pair, 117 certified).
+// rows: those of 65 / 103 / 203 / 403 sources go pair by pair from 510 / 650 / 1070 / 2160 sinks (an
+// evaluation of 65 massive bodies and 5000 test particles: 85 us in rows, 23 pair by pair, 68
+// certified; an RKF7(8) attempt of 5 disks of 403 bodies 974 us in rows, 1088 pair by pair, of 12 1971
+// and 1736), certified from some 180 000 / 21 000 / 6300 / 2600 (203 and 20 000: 189 us pair by pair, 117
+// certified; 12 disks of 303 bodies 868 us pair by pair, 1219 certified, of 30 2071 and 1360).
 enum Fp64Form { FP64_FORM_ROWS, FP64_FORM_PAIRPAR, FP64_FORM_CERT };
 constexpr int64_t FP64_ROW_PAIRS = 2250000;
-inline bool fp64_wide(int64_t rows, int64_t pairs)  // rows > 400 + 2.8 sources
+inline bool fp64_wide(int64_t rows, int64_t pairs)
 {
-    return 5 * (rows - 400) * rows > 14 * pairs;
+    const int64_t src = rows > 0 ? pairs / rows : 0;
+    return 1000 * rows > 300000 + 3000 * src + 4 * src * src;
 }
 inline Fp64Form fp64_block_form(int64_t rows, int64_t pairs)
 {
     if (!fp64_wide(rows, pairs)) return pairs <= FP64_ROW_PAIRS ? FP64_FORM_ROWS : FP64_FORM_CERT;
-    return pairs - 60 * rows <= 700000 ? FP64_FORM_PAIRPAR : FP64_FORM_CERT;  // rows (sources - 60)
+    return pairs - 60 * rows <= 900000 ? FP64_FORM_PAIRPAR : FP64_FORM_CERT;  // rows (sources - 60)
 }
 
 // The sinks S of a pair-parallel CTA for the blocks added: 256 threads take four terms each of S x
 // 1024 / S pairs at a time, `resident` CTAs on each of n_sm SMs.  The S of the least waves x steps (a
-// CTA starts and sums for as long as two steps of terms take; half a wave's rounding counts: an
+// CTA starts and sums for as long as two steps of terms take; two thirds of a wave's rounding count: an
 // evaluation of 203 massive bodies and 2000 test particles takes 39 us with 8 and 54 with 16, with
 // 5000 82 and 73; 64 disks of 103 bodies 565 us an attempt with 8, 529 with 16, 661 with 32).
 struct PairparSinks {
@@ -57,7 +59,7 @@ struct PairparSinks {
         for (int k = 0; k < 4; k++) {
             if (ctas[k] <= 0.0) continue;
             const double waves = ctas[k] / ((double)resident * std::max(n_sm, 1));
-            const double cost = (std::ceil(waves) + std::max(1.0, waves)) * steps[k] / ctas[k];
+            const double cost = (2.0 * std::ceil(waves) + std::max(1.0, waves)) * steps[k] / ctas[k];
             if (least < 0.0 || cost < least) {
                 least = cost;
                 s = S[k];

@@ -20,17 +20,19 @@ int main()
             printf("%ld rows of %ld: form %d, not %d\n", rows, sources, (int)got, (int)want);
         }
     };
-    // sinks x sources: rows up to 400 + 2.8 sources ...
-    for (long src : {65, 103, 203, 403}) {
-        const long line = (long)(400 + 2.8 * (double)src);
+    // sinks x sources: rows up to 300 + 3 sources + sources^2 / 250 ...
+    for (long src : {65, 103, 203, 303, 403}) {
+        const long line = (300000 + 3000 * src + 4 * src * src) / 1000;
         expect(1, src, FP64_FORM_ROWS);
         expect(line, src, FP64_FORM_ROWS);
         expect(line + 1, src, FP64_FORM_PAIRPAR);
-        const long last = 700000 / (src - 60);  // ... pair by pair up to rows (sources - 60) = 700 000
+        const long last = 900000 / (src - 60);  // ... pair by pair up to rows (sources - 60) = 900 000
         expect(last, src, FP64_FORM_PAIRPAR);
         expect(last + 1, src, FP64_FORM_CERT);
         expect(1000000, src, FP64_FORM_CERT);
     }
+    expect(3016, 603, FP64_FORM_ROWS);
+    expect(5000, 603, FP64_FORM_CERT);
     expect(1500, 1500, FP64_FORM_ROWS);  // square blocks by their pairs
     expect(1501, 1501, FP64_FORM_CERT);
     expect(131074, 131074, FP64_FORM_CERT);
@@ -63,7 +65,7 @@ int main()
                         steps += (m * q + 255) / 256;
                     }
                     const double waves = (double)ctas / 456.0;
-                    const double cost = (std::ceil(waves) + (waves > 1.0 ? waves : 1.0)) * (double)steps;
+                    const double cost = (2.0 * std::ceil(waves) + (waves > 1.0 ? waves : 1.0)) * (double)steps;
                     if (cost < least) {
                         least = cost;
                         want = q;

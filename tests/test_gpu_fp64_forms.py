@@ -24,9 +24,9 @@ def _disk(si, pl, tp, seed=1):
 
 
 def _sizes():
-    # sinks around 400 + 2.8 sources, tiles of 4 to 32 sinks with one over, sources around the tiles' 32 to 256
-    return [(62, 0, 582), (62, 0, 583), (62, 1501, 0), (62, 0, 4801), (70, 700, 701), (125, 0, 1537), (126, 2000, 33),
-            (200, 0, 969), (200, 967, 968), (200, 0, 4895), (200, 0, 4896), (253, 0, 1700), (254, 1111, 0), (400, 0, 1999)]
+    # sinks on both sides of the line to rows, tiles of 4 to 32 sinks with one over, sources around the tiles' 32 to 256
+    return [(62, 0, 511), (62, 0, 512), (62, 1501, 0), (62, 0, 4801), (70, 700, 701), (125, 0, 1537), (126, 2000, 33),
+            (200, 0, 1073), (200, 1074, 1075), (200, 0, 6293), (200, 0, 6294), (253, 0, 1700), (254, 1333, 0), (400, 0, 2160)]
 
 
 @pytest.mark.parametrize("si,pl,tp", _sizes())
@@ -62,6 +62,20 @@ def test_events_match_oracle(gpulib, si, pl, tp):
         for f in T.EVENT.names:
             assert a[f] == b[f], (f, a, b)
     for a, b in zip(sg[:2], so[:2]):
+        for f in "xyz":
+            assert H.same(a[f], b[f]), f
+
+
+def test_steps_with_all_forms(gpulib):
+    """RKF7(8) attempts from a graph, with rows, a block pair by pair and a certified one on two streams."""
+    d, thr = _disk(100, 2000, 1200), bodies.thresholds()
+    got = []
+    for s in (lib.System(d, thr), pyoracle.OracleSystem(d, thr)):
+        s.set_integrator(T.INT_RKF78, 1.0, True, 1e-10)
+        s.set_event_options(hill_factor=3.0)
+        s.advance(1e9, max_steps=3)
+        got.append(s.state(internal=True))
+    for a, b in zip(got[0][:2], got[1][:2]):
         for f in "xyz":
             assert H.same(a[f], b[f]), f
 
