@@ -458,12 +458,12 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 //
 // A component whose sum is small beside its terms (a sink close to the disk's plane: its z sum)
 // has few certain terms.  Once more than an eighth of an epoch's pairs are uncertain in it, or it
-// has left its binade in four epochs, the sink goes to a list of rows, the component is dropped
+// has left its binade in four epochs (in one where the rows are short), the sink goes to a list of rows, the component is dropped
 // here, and grav_fp64_rows adds it from exact terms.  A sink outside the grid goes there whole, with
 // its event tests: its exact pairs in one warp would be the last thing running (one body at 100 AU
 // in a disk of 8003 bodies with collisions on: an RKF7(8) attempt 21.7 ms, 8.9 without it).  So does
-// a sink with an eighth of its pairs flagged that no failing component explains (sources outside the
-// grid, wide screens), whose exact pairs cost eleven times the row kernel's, and so do all, once
+// a sink whose flagged pairs no failing component explains (sources outside the grid, wide screens) and
+// are more than an eighth: an exact pair here costs eleven of the row kernel's.  And so do all, once
 // three quarters of the sinks begun have rows in the list (a row costs what three or four
 // sinks do here); and a sink whose sums are all left to the row kernel is done here.  An RK4 step of 8003
 // bodies with collisions on, of them 10 / 30 % out to thousands of AU 22.2 / 30.3 -> 9.8 / 10.6 ms, 10 %
@@ -643,6 +643,8 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     fetch(j0, 0);
     fetch(j0, 1);
     int n_redo = 0, n_exact = 0;  // n_exact: this lane's flagged pairs that no failing component explains
+    // epochs a sum may leave its binade in: taken again, one costs up to its pairs exactly, a row an eighth of its own
+    const int redo_most = min(4, 1 + (tile.src_end - tile.src_begin) / (8 * EPOCH));
     int tests = outside ? j_head : tile.src_end;  // the first source whose event tests are the row kernel's
     unsigned live = act & ~__ballot_sync(ALL, outside) & SINKS;  // sinks with sums left here (or events to find)
     unsigned listed = act & SINKS & ~live;                       // sinks with a row in the list
@@ -780,11 +782,13 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
             int n = n_exact;
             for (int off = SW; off < 32; off <<= 1) n += __shfl_xor_sync(ALL, n, off);
             const bool many = __any_sync(ALL, begun >= 512u && 4ull * rows > 3ull * begun);  // (by every lane)
-            whole = many || (n > 32 && 8 * n > passed + nj);
+            // as many to come as up to here, against a row's cost: that of an eighth of its pairs, or of 50
+            const long long left = tile.src_end - (j0 + nj), all = max(400, tile.src_end - tile.src_begin);
+            whole = many || (n > 32 && 8 * n * left > (passed + nj) * all);
         }
         if (owner && !deferred && (act >> s & 1)) {
             n_redo += ok ? 0 : (acc == 0.0 ? 4 : 1);  // (a sum that is zero so far will hover)
-            deferred = deferred || whole || (int)(fail >> (10 * c) & 1023u) * 8 > nj || n_redo >= 4;
+            deferred = deferred || whole || (int)(fail >> (10 * c) & 1023u) * 8 > nj || n_redo >= redo_most;
             ok = ok || deferred;
         }
         // sums (bit c SW + s) whose epoch is taken slice by slice

@@ -21,7 +21,7 @@ namespace redgb {
 // rows: those of 65 / 103 / 203 / 403 sources go pair by pair from 510 / 650 / 1070 / 2160 sinks (an
 // evaluation of 65 massive bodies and 5000 test particles: 85 us in rows, 23 pair by pair, 68
 // certified; an RKF7(8) attempt of 5 disks of 403 bodies 974 us in rows, 1088 pair by pair, of 12 1971
-// and 1736), certified from some 180 000 / 21 000 / 6300 / 2600 (203 and 20 000: 189 us pair by pair, 117
+// and 1736), certified from some 240 000 / 28 000 / 8400 / 3500 (203 and 20 000: 189 us pair by pair, 117
 // certified; 12 disks of 303 bodies 868 us pair by pair, 1219 certified, of 30 2071 and 1360).
 enum Fp64Form { FP64_FORM_ROWS, FP64_FORM_PAIRPAR, FP64_FORM_CERT };
 constexpr int64_t FP64_ROW_PAIRS = 2250000;
@@ -33,7 +33,7 @@ inline bool fp64_wide(int64_t rows, int64_t pairs)
 inline Fp64Form fp64_block_form(int64_t rows, int64_t pairs)
 {
     if (!fp64_wide(rows, pairs)) return pairs <= FP64_ROW_PAIRS ? FP64_FORM_ROWS : FP64_FORM_CERT;
-    return pairs - 60 * rows <= 900000 ? FP64_FORM_PAIRPAR : FP64_FORM_CERT;  // rows (sources - 60)
+    return pairs - 60 * rows <= 1200000 ? FP64_FORM_PAIRPAR : FP64_FORM_CERT;  // rows (sources - 60)
 }
 
 // The sinks S of a pair-parallel CTA for the blocks added: 256 threads take four terms each of S x

@@ -26,7 +26,7 @@ int main()
         expect(1, src, FP64_FORM_ROWS);
         expect(line, src, FP64_FORM_ROWS);
         expect(line + 1, src, FP64_FORM_PAIRPAR);
-        const long last = 900000 / (src - 60);  // ... pair by pair up to rows (sources - 60) = 900 000
+        const long last = 1200000 / (src - 60);  // ... pair by pair up to rows (sources - 60) = 1 200 000
         expect(last, src, FP64_FORM_PAIRPAR);
         expect(last + 1, src, FP64_FORM_CERT);
         expect(1000000, src, FP64_FORM_CERT);

@@ -26,7 +26,7 @@ def _disk(si, pl, tp, seed=1):
 def _sizes():
     # sinks on both sides of the line to rows, tiles of 4 to 32 sinks with one over, sources around the tiles' 32 to 256
     return [(62, 0, 511), (62, 0, 512), (62, 1501, 0), (62, 0, 4801), (70, 700, 701), (125, 0, 1537), (126, 2000, 33),
-            (200, 0, 1073), (200, 1074, 1075), (200, 0, 6293), (200, 0, 6294), (253, 0, 1700), (254, 1333, 0), (400, 0, 2160)]
+            (200, 0, 1073), (200, 1074, 1075), (200, 0, 8391), (200, 0, 8392), (253, 0, 1700), (254, 1333, 0), (400, 0, 2160)]
 
 
 @pytest.mark.parametrize("si,pl,tp", _sizes())
