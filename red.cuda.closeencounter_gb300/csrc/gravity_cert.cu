@@ -466,8 +466,8 @@ __global__ void __launch_bounds__(PREP_NT) cert_prep_kernel(CertPrepArgs a)
 // are more than an eighth: an exact pair here costs eleven of the row kernel's.  And so do all, once
 // three quarters of the sinks begun have rows in the list (a row costs what three or four
 // sinks do here); and a sink whose sums are all left to the row kernel is done here.  An RK4 step of 8003
-// bodies with collisions on, of them 10 / 30 % out to thousands of AU 22.2 / 30.3 -> 9.8 / 10.6 ms, 10 %
-// above an otherwise flat disk 29.8 -> 11.8 ms (every pair on the FP64 pipe: 9.7 ms).
+// bodies with collisions on, of them 10 / 30 % out to thousands of AU 22.2 / 30.3 -> 9.8 / 10.7 ms, 10 %
+// above an otherwise flat disk 29.8 -> 10.2 ms (every pair on the FP64 pipe: 9.7 ms).
 template <int SW, bool SCREEN>
 __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     grav_fp64_cert(GravArgs g, CertRows cr)
@@ -642,6 +642,7 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
     };
     fetch(j0, 0);
     fetch(j0, 1);
+    int again = 0;                // times the epoch has been taken again for flagged sinks
     int n_redo = 0, n_exact = 0;  // n_exact: this lane's flagged pairs that no failing component explains
     // epochs a sum may leave its binade in: taken again, one costs up to its pairs exactly, a row an eighth of its own
     const int redo_most = min(4, 1 + (tile.src_end - tile.src_begin) / (8 * EPOCH));
@@ -695,6 +696,34 @@ __global__ void __launch_bounds__(32 * CERT_WARPS, 16 / CERT_WARPS)
             deferred = deferred || (most && owner);
             if (most) flags = 0u;
         }
+        // with event tests: a sink with most of its pairs flagged loses its smallest sum, which is the one they
+        // are uncertain in as a rule, or, if that does not help, goes to the row kernel whole; and the warp
+        // takes the epoch again.  (Their exact pairs cost eleven times the row's: an RKF7(8) attempt of 30 disks
+        // of 303 bodies, a tenth of them above an otherwise flat disk, 9.1 ms, 4.1 so; of ordinary ones
+        // 1.60 and 1.33 ms.)
+        if (SCREEN && __any_sync(ALL, 2 * __popc(flags) > cnt)) {  // (one lane of such a sink has most of its own)
+            int n = __popc(flags);
+            for (int off = SW; off < 32; off <<= 1) n += __shfl_xor_sync(ALL, n, off);
+            const bool most = n > 32 && 2 * n > nj && (live >> s & 1u);
+            const int size = owner && !deferred && acc != 0.0 ? (int)((xf::dbits(acc) >> 52) & 0x7ff) : 4096;
+            const int s0 = __shfl_sync(ALL, size, s), s1 = __shfl_sync(ALL, size, SW + s), s2 = __shfl_sync(ALL, size, 2 * SW + s);
+            const int least = s2 <= min(s0, s1) ? 2 : (s1 <= s0 ? 1 : 0);  // z first: a disk's plane
+            if (__any_sync(ALL, most)) {
+                const bool whole = most && again > 0;
+                if (owner && most && (whole || c == least)) deferred = true;
+                if (whole) tests = j0;
+                live &= ~__ballot_sync(ALL, whole);
+                again++;
+                publish();
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncwarp();
+                fetch(j0, 0);
+                fetch(j0, 1);
+                j0 -= EPOCH;
+                continue;
+            }
+        }
+        again = 0;
         // each high and low integer carries MAGIC's bits
         const unsigned nb = (unsigned)n_done * MAGIC_BITS;
         long long px = (long long)(int)(sum.hx - nb) * 65536 + (int)(sum.lx - nb);
