@@ -22,7 +22,7 @@ namespace redgb {
 // evaluation of 65 massive bodies and 5000 test particles: 85 us in rows, 23 pair by pair, 68
 // certified; an RKF7(8) attempt of 5 disks of 403 bodies 974 us in rows, 1088 pair by pair, of 12 1971
 // and 1736), certified from some 240 000 / 28 000 / 8400 / 3500 (203 and 20 000: 189 us pair by pair, 117
-// certified; 12 disks of 303 bodies 868 us pair by pair, 1219 certified, of 30 2071 and 1360).
+// certified; 12 disks of 303 bodies 868 us pair by pair, 1219 certified, of 30 2071 and 1330).
 enum Fp64Form { FP64_FORM_ROWS, FP64_FORM_PAIRPAR, FP64_FORM_CERT };
 constexpr int64_t FP64_ROW_PAIRS = 2250000;
 inline bool fp64_wide(int64_t rows, int64_t pairs)
